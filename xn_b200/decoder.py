@@ -11,11 +11,10 @@ a CUDA graph.  Buffers are allocated once in the constructor.
 """
 from __future__ import annotations
 
-import math
-
 import torch
 
-from ._lib import BF16, check, lib
+from . import _host
+from ._lib import lib
 
 
 class DecoderStack:
@@ -77,66 +76,13 @@ class DecoderStack:
         self.pos = torch.full((B,), context - 1, dtype=torch.int64, device=device)
         self.mask = None  # optional f32 [B, context] additive mask
 
-    # -- helpers -------------------------------------------------------------------------------
-    def _s(self):
-        return torch.cuda.current_stream().cuda_stream
-
-    def _linear(self, y, wq_ws, m, n, k):
-        wq, ws = wq_ws
-        check(lib().xn_mm_linear_fp8_pieces(y.data_ptr(), self.hi.data_ptr(),
-                                            self.lo.data_ptr() if self.variant == 0 else None, self.xs.data_ptr(),
-                                            wq.data_ptr(), ws.data_ptr(), m, n, k, self._s()))
-
-    def _lo(self):
-        return self.lo.data_ptr() if self.variant == 0 else None
-
     def step(self, x: torch.Tensor) -> torch.Tensor:
-        """x: [streams, d_model] bf16 (the embedded token of every stream). Returns the stack's output."""
-        L, B, d, H, hid, ctx = lib(), self.B, self.d, self.H, self.hid, self.ctx
-        s = self._s()
-        cur = x
-        for li, lay in enumerate(self.layers):
-            if li == 0:  # later layers get their pieces from the fused add + norm that ends the previous layer
-                check(L.xn_mm_rms_norm_split_e4m3(self.hi.data_ptr(), self._lo(), self.xs.data_ptr(), None, cur.data_ptr(),
-                                                  lay["norm1"].data_ptr(), BF16, B, d, self.eps, s))
-            self._linear(self.qkv, lay["in_proj"], B, 3 * d, d)
-            q, kn, vn = self.qkv.data_ptr(), self.qkv.data_ptr() + 2 * d, self.qkv.data_ptr() + 4 * d
-            if self.attention == "separate":
-                check(L.xn_mm_kv_append2(BF16, lay["k"].data_ptr(), lay["v"].data_ptr(), kn, vn, 3 * d, self.pos.data_ptr(), B, H,
-                                         ctx, 128, s))
-                # attention over the cache; the merge of the context slices also writes the e4m3 pieces of the output row
-                check(L.xn_mm_decode_attention_split_e4m3(self.hi.data_ptr(), self._lo(), self.xs.data_ptr(),
-                                                          self.attn.data_ptr(), q, 3 * d, lay["k"].data_ptr(),
-                                                          lay["v"].data_ptr(),
-                                                          self.mask.data_ptr() if self.mask is not None else None, B, H, ctx,
-                                                          128, 1.0 / math.sqrt(128.0), self.attn_ws.data_ptr(),
-                                                          self.attn_ws_bytes, s))
-            else:
-                # append the new key / value rows, attend over the cache, merge the context slices and write the e4m3
-                # pieces of the output row
-                check(L.xn_mm_decode_attention_append_e4m3(self.hi.data_ptr(), self._lo(), self.xs.data_ptr(),
-                                                           self.attn.data_ptr(), q, kn, vn, 3 * d, lay["k"].data_ptr(),
-                                                           lay["v"].data_ptr(), self.pos.data_ptr(),
-                                                           self.mask.data_ptr() if self.mask is not None else None, B, H, ctx,
-                                                           128, 1.0 / math.sqrt(128.0),
-                                                           1 if self.attention == "fused_one_launch" else 0,
-                                                           self.attn_ws.data_ptr(), self.attn_ws_bytes, s))
-            self._linear(self.proj, lay["out_proj"], B, d, d)
-            check(L.xn_mm_add_rms_norm_split_e4m3(self.hi.data_ptr(), self._lo(), self.xs.data_ptr(), self.x_mid.data_ptr(),
-                                                  cur.data_ptr(), self.proj.data_ptr(), lay["norm2"].data_ptr(), BF16, B, d,
-                                                  self.eps, s))
-            self._linear(self.h, lay["linear_in"], B, 2 * hid, d)
-            check(L.xn_mm_silu_mul_split_e4m3(self.hi.data_ptr(), self._lo(), self.xs.data_ptr(), self.h.data_ptr(), BF16,
-                                              B, hid, s))
-            self._linear(self.proj, lay["linear_out"], B, d, hid)
-            if li + 1 < len(self.layers):  # x_out = x_mid + proj, pieces of the next layer's norm1(x_out)
-                check(L.xn_mm_add_rms_norm_split_e4m3(self.hi.data_ptr(), self._lo(), self.xs.data_ptr(),
-                                                      self.x_out.data_ptr(), self.x_mid.data_ptr(), self.proj.data_ptr(),
-                                                      self.layers[li + 1]["norm1"].data_ptr(), BF16, B, d, self.eps, s))
-            else:
-                check(L.xn_mm_add(BF16, self.x_out.data_ptr(), self.x_mid.data_ptr(), self.proj.data_ptr(), B * d, s))
-            cur = self.x_out
-        return self.x_out
+        """x: [streams, d_model] bf16 (the embedded token of every stream). Returns the stack's output.
+
+        Per layer: [norm1 + split] -> in_proj -> cache append, attention, merge + split -> out_proj -> add + norm2 + split
+        -> linear_in -> silu * mul + split -> linear_out -> add + next norm1 + split; the walk over the layers is native
+        (csrc/host/binding.cpp, decoder_step)."""
+        return _host.decoder_step(self, x)
 
     def bytes_per_step(self) -> dict:
         d, hid, B, ctx, H = self.d, self.hid, self.B, self.ctx, self.H

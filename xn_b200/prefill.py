@@ -256,6 +256,9 @@ class PrefillStack:
 
     def forward(self, x):
         """x: [tokens, d_model] bf16, the same on every rank.  Returns the stack's [tokens, d_model] output (on every rank)."""
+        if self.world == 1 and self.fused_attention:  # nothing to exchange: the walk over the layers is native
+            from . import _host
+            return _host.prefill_forward(self, x)
         import math
 
         from ._lib import BF16, check, lib
@@ -271,9 +274,8 @@ class PrefillStack:
             qkv4 = self.qkv.view(T, 3, Hl, 128)
             q, k, v = (qkv4[:, j].transpose(0, 1) for j in range(3))      # [Hl, T, 128] views, rows 3*dl apart
             if self.fused_attention:
-                # one kernel for the rank's heads: scores and probabilities never leave the SM (a single rank owns
-                # every head and writes the rows the out projection reads: nothing to exchange)
-                attention_prefill_(self.attn_full.t if self.world == 1 else self.attn_rows, q, k, v, 1.0 / math.sqrt(128.0))
+                # one kernel for the rank's heads: scores and probabilities never leave the SM
+                attention_prefill_(self.attn_rows, q, k, v, 1.0 / math.sqrt(128.0))
             else:
                 # q.k^T, one launch for the rank's heads; tiles beyond the causal horizon are skipped
                 matmul_causal_(self.scores, q, k, True, 1, 0)
@@ -282,8 +284,7 @@ class PrefillStack:
                 # p.v, [T, 128] right-hand side per head; every row tile stops at its horizon
                 matmul_causal_(self.attn_l, self.scores, v, False, 2, 0)
             if self.fused_attention:
-                if self.world > 1:
-                    self._gather(self.attn_full, self.attn_rows, d, 1)
+                self._gather(self.attn_full, self.attn_rows, d, 1)
             else:
                 self._gather(self.attn_full, self.attn_l, d, Hl)
             check(L.xn_mm_split_rows_e4m3(self.hi.data_ptr(), self._lo(), self.xs.data_ptr(), self.attn_full.t.data_ptr(), BF16,
