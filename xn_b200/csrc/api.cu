@@ -114,6 +114,16 @@ static int gemm_dispatch(xn_dtype dtype, void *dst, const void *lhs, size_t lhs_
     if (h16_fits && lhs_b == 1 && n >= 64 && lhs_cs == 1 && rhs_rs == 1 && dst_cs == 1 && k % 8 == 0 &&
         lhs_rs % 8 == 0 && rhs_cs % 8 == 0 && aligned(l, 16) && aligned(r, 16) && k <= 0x7fffffff)
         return launch_gemv_h16(dtype, dst, l, r, m, n, k, dst_rs, lhs_rs, rhs_cs, (cudaStream_t)stream);
+    // The same with one right-hand side per batch entry (per-codebook weights, the keys of a decode step).
+    if (tn16_ok && m <= 16 && lhs_b > 1 && lhs_b_stride % 8 == 0 && rhs_b_stride % 8 == 0 && gemv_h16_batched_fits(m, n, k, lhs_b))
+        return launch_gemv_h16_batched(dtype, dst, l, r, m, n, k, lhs_b, lhs_b_stride, rhs_b_stride, dst_rs, lhs_rs, rhs_cs,
+                                       (cudaStream_t)stream);
+    // Up to 16 rows against a row-major [k, n] right-hand side, any batch count and any lhs row pitch.
+    const bool kn16_rhs = dtype != XN_F32 && lhs_cs == 1 && rhs_cs == 1 && dst_cs == 1 && rhs_rs % 8 == 0 && rhs_rs >= n && aligned(r, 16) &&
+                          (lhs_b == 1 || rhs_b_stride % 8 == 0);
+    if (kn16_rhs && m <= 16 && !causal && gemv_kn16_fits(m, n, k, lhs_b))
+        return launch_gemv_kn16(dtype, dst, l, r, m, n, k, lhs_b, lhs_b_stride, rhs_b_stride, dst_rs, lhs_rs, rhs_rs,
+                                (cudaStream_t)stream);
     // Decode-sized matmul_t (m <= 16, both operands k-contiguous): the weight-streaming kernel with exact f32
     // products, for all three element types and any batch count.
     {
@@ -169,6 +179,13 @@ static int gemm_dispatch(xn_dtype dtype, void *dst, const void *lhs, size_t lhs_
                                        (rhs_b_stride >= k * rhs_rs || (rhs_b_stride >= n && lhs_b * rhs_b_stride <= rhs_rs)))))
             return launch_gemm_kn_16bit(dtype, dst, l, r, m, n, k, lhs_rs, rhs_rs, dst_rs, lhs_b, lhs_b_stride, rhs_b_stride,
                                         (cudaStream_t)stream, causal == 2 ? 2 : 0, causal_off);
+        // rows of lhs off 16-byte boundaries: copied to a pitch TMA can address first
+        const size_t most = (size_t)1 << 30;
+        if (!kn_off && kn16_rhs && !causal && (k % 8 || lhs_rs % 8 || lhs_b_stride % 8 || !aligned(l, 16)) && n >= 2 && m <= most && n <= most &&
+            k <= most && dst_rs <= 0x7fffffff && lhs_b <= 0x7fffffff &&
+            (lhs_b == 1 || rhs_b_stride >= k * rhs_rs || (rhs_b_stride >= n && lhs_b * rhs_b_stride <= rhs_rs)))
+            return launch_gemm_kn_repitched(dtype, dst, l, r, m, n, k, lhs_b, lhs_b_stride, rhs_b_stride, dst_rs, lhs_rs, rhs_rs,
+                                            (cudaStream_t)stream);
     }
     if (causal == 2)
         return fail(XN_ERR_UNSUPPORTED, "gemm_causal (values): needs 16-bit elements, an n-contiguous right-hand side and "

@@ -81,6 +81,24 @@ int ensure_dynamic_smem(const void *kernel, int *slot, size_t bytes);
         if (_rc) return _rc;                                                                  \
     } while (0)
 
+// Launch with programmatic stream serialization: the kernel may start while its predecessor drains, and touches nothing
+// the predecessor wrote before its own griddepcontrol.wait.
+template <typename... P, typename... A>
+int launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    XN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
+    return XN_OK;
+}
+
 // Element widening / narrowing (round to nearest even), the same conversions crate `half`
 // performs for the reference (xn-core/src/dtype.rs:92-131).
 __device__ __forceinline__ float to_f32(float v) { return v; }
@@ -130,6 +148,14 @@ int launch_gemm_generic(xn_dtype dt, void *dst, const void *lhs, const void *rhs
 bool gemv_h16_single_chunk(size_t m, size_t k);
 int launch_gemv_h16(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k, size_t dst_rs,
                     size_t lhs_rs, size_t rhs_cs, cudaStream_t st);
+bool gemv_h16_batched_fits(size_t m, size_t n, size_t k, size_t batch);
+int launch_gemv_h16_batched(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k, size_t batch,
+                            size_t lhs_bs, size_t rhs_bs, size_t dst_rs, size_t lhs_rs, size_t rhs_cs, cudaStream_t st);
+bool gemv_kn16_fits(size_t m, size_t n, size_t k, size_t batch);
+int launch_gemv_kn16(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k, size_t batch,
+                     size_t lhs_bs, size_t rhs_bs, size_t dst_rs, size_t lhs_rs, size_t rhs_rs, cudaStream_t st);
+int launch_gemm_kn_repitched(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k, size_t batch,
+                             size_t lhs_bs, size_t rhs_bs, size_t dst_rs, size_t lhs_rs, size_t rhs_rs, cudaStream_t st);
 int launch_gemv_f32x3(float *dst, const float *lhs, const float *rhs, size_t m, size_t n, size_t k, size_t dst_rs,
                       size_t lhs_rs, size_t rhs_cs, cudaStream_t st);
 int launch_gemv_dense(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k,
