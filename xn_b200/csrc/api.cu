@@ -109,18 +109,29 @@ static int gemm_dispatch(xn_dtype dtype, void *dst, const void *lhs, size_t lhs_
     const bool tn16_ok = dtype != XN_F32 && lhs_cs == 1 && rhs_rs == 1 && dst_cs == 1 && k % 8 == 0 && lhs_rs % 8 == 0 &&
                          rhs_cs % 8 == 0 && aligned(l, 16) && aligned(r, 16) && m <= 0x7fffffff && n <= 0x7fffffff &&
                          k <= 0x7fffffff && dst_rs <= 0x7fffffff;
-    // up to 16 rows with k too long for the weight-streaming kernel's staged activations: tensor-memory skinny form
-    const bool long_k_skinny = tn16_ok && m <= 16 && !h16_fits && n >= 256 && lhs_b == 1;
-    if (h16_fits && lhs_b == 1 && n >= 64 && lhs_cs == 1 && rhs_rs == 1 && dst_cs == 1 && k % 8 == 0 &&
-        lhs_rs % 8 == 0 && rhs_cs % 8 == 0 && aligned(l, 16) && aligned(r, 16) && k <= 0x7fffffff)
-        return launch_gemv_h16(dtype, dst, l, r, m, n, k, dst_rs, lhs_rs, rhs_cs, (cudaStream_t)stream);
+    // Up to 16 rows the mma.sync kernel streams a weight without the tensor-memory kernel's fixed cost, except where the
+    // latter's split along k pays: a long k, or 9 to 16 rows (two column groups) while the channels leave SMs to split over.
+    // us, streaming / tensor memory, bf16: 1 x 4096 x 4096 8.0 / 8.9, 1 x 22528 x 4096 28.3 / 31.0, 1 x 4096 x 11264
+    // 20.3 / 17.3; 16 x 4096 x 4096 10.7 / 9.3, 16 x 12288 x 4096 20.9 / 19.8, 16 x 22528 x 4096 31.4 / 33.4.
+    const bool narrow = (n + 127) / 128 <= (size_t)sm_count();
+    const bool skinny16 = tn16_ok && lhs_b == 1 && !causal && gemm_skinny_wanted(m, n, k) &&
+                          (m > 16 || !h16_fits || (n >= 256 && narrow && (m > 8 || (k >= 8192 && (n + 63) / 64 <= (size_t)sm_count()))));
+    if (skinny16)
+        return launch_skinny_16bit(dtype, dst, l, r, take_fused_col_bias(), m, n, k, lhs_rs, rhs_cs, dst_rs, 1, 0, 0, 0, false,
+                                   (cudaStream_t)stream);
+    if (h16_fits && lhs_b == 1 && n >= 64 && tn16_ok)
+        return launch_gemv_h16(dtype, dst, l, r, m, n, k, dst_rs, lhs_rs, rhs_cs, take_fused_col_bias(), (cudaStream_t)stream);
     // The same with one right-hand side per batch entry (per-codebook weights, the keys of a decode step).
     if (tn16_ok && m <= 16 && lhs_b > 1 && lhs_b_stride % 8 == 0 && rhs_b_stride % 8 == 0 && gemv_h16_batched_fits(m, n, k, lhs_b))
         return launch_gemv_h16_batched(dtype, dst, l, r, m, n, k, lhs_b, lhs_b_stride, rhs_b_stride, dst_rs, lhs_rs, rhs_cs,
                                        (cudaStream_t)stream);
-    // Up to 16 rows against a row-major [k, n] right-hand side, any batch count and any lhs row pitch.
+    // A row-major [k, n] right-hand side: one weight for up to 64 (128) rows on the tensor-memory kernel with the weight as its
+    // MN-major operand; up to 16 rows with any batch count and any lhs row pitch on the streaming kernel.
     const bool kn16_rhs = dtype != XN_F32 && lhs_cs == 1 && rhs_cs == 1 && dst_cs == 1 && rhs_rs % 8 == 0 && rhs_rs >= n && aligned(r, 16) &&
                           (lhs_b == 1 || rhs_b_stride % 8 == 0);
+    if (kn16_rhs && lhs_b == 1 && !causal && k % 8 == 0 && lhs_rs % 8 == 0 && aligned(l, 16) && dst_rs <= 0x7fffffff &&
+        gemm_skinny_wanted(m, n, k))
+        return launch_skinny_16bit(dtype, dst, l, r, nullptr, m, n, k, lhs_rs, rhs_rs, dst_rs, 1, 0, 0, 0, true, (cudaStream_t)stream);
     if (kn16_rhs && m <= 16 && !causal && gemv_kn16_fits(m, n, k, lhs_b))
         return launch_gemv_kn16(dtype, dst, l, r, m, n, k, lhs_b, lhs_b_stride, rhs_b_stride, dst_rs, lhs_rs, rhs_rs,
                                 (cudaStream_t)stream);
@@ -128,7 +139,7 @@ static int gemm_dispatch(xn_dtype dtype, void *dst, const void *lhs, size_t lhs_
     // products, for all three element types and any batch count.
     {
         const size_t v = 16 / es;
-        if (m <= 16 && !long_k_skinny && lhs_cs == 1 && rhs_rs == 1 && dst_cs == 1 && k % v == 0 && lhs_rs % v == 0 && rhs_cs % v == 0 &&
+        if (m <= 16 && lhs_cs == 1 && rhs_rs == 1 && dst_cs == 1 && k % v == 0 && lhs_rs % v == 0 && rhs_cs % v == 0 &&
             (lhs_b == 1 || (lhs_b_stride % v == 0 && rhs_b_stride % v == 0)) && aligned(l, 16) && aligned(r, 16)) {
             // f32, one batch, k a multiple of 32, a weight worth streaming: the tensor-core 3xTF32 form
             // (products to ~1e-6 relative; XN_MM_F32_EXACT=1 keeps the exact-product FFMA kernel)
@@ -160,7 +171,7 @@ static int gemm_dispatch(xn_dtype dtype, void *dst, const void *lhs, size_t lhs_
     // Linear::forward's form with 16-bit elements -- both operands k-contiguous, rows of dst
     // contiguous -- goes to the tcgen05 kernel when TMA can address it (16-byte pitches and bases).
     // The strided-batched / grouped form (lhs_b > 1 with per-batch weights) is one launch as well.
-    if (tn16_ok && (m > 16 || long_k_skinny) &&
+    if (tn16_ok && m > 16 &&
         (lhs_b == 1 || (lhs_b <= 0x7fffffff && lhs_b_stride % 8 == 0 && rhs_b_stride % 8 == 0 && rhs_b_stride != 0 &&
                         lhs_b_stride != 0)))
         return launch_gemm_tn_16bit(dtype, dst, l, r, m, n, k, lhs_rs, rhs_cs, dst_rs, lhs_b, lhs_b_stride, rhs_b_stride,

@@ -84,7 +84,7 @@ int ensure_dynamic_smem(const void *kernel, int *slot, size_t bytes);
 // Launch with programmatic stream serialization: the kernel may start while its predecessor drains, and touches nothing
 // the predecessor wrote before its own griddepcontrol.wait.
 template <typename... P, typename... A>
-int launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+int launch_kernel(bool dependent, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -94,9 +94,13 @@ int launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cud
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = dependent && pdl_enabled() ? 1 : 0;
     XN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...));
     return XN_OK;
+}
+template <typename... P, typename... A>
+int launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+    return launch_kernel(true, kern, grid, block, smem, st, args...);
 }
 
 // Element widening / narrowing (round to nearest even), the same conversions crate `half`
@@ -131,6 +135,41 @@ __device__ __forceinline__ uint4 ldg_stream(const void *p) {
     return v;
 }
 
+// Kernels launched with launch_dependent() start with this: the next kernel in the stream may begin its own set-up (and
+// fetch what is static, a linear's weights above all) while this one runs, and nothing is touched before the previous
+// one has finished.
+__device__ __forceinline__ void dependent_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// Loads of what the previous kernel in the stream wrote, for kernels that may be resident while it still runs: through
+// L2, and never moved ahead of the wait above (a load through a const __restrict__ pointer or __ldg may be, and may be
+// served from a line that a neighbour CTA of an earlier kernel left in L1).
+__device__ __forceinline__ uint4 ld_act128(const void *p) {
+    uint4 v;
+    asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ float ld_act_f32(const float *p) {
+    float v;
+    asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned short ld_act_u16(const void *p) {
+    unsigned short v;
+    asm volatile("ld.global.cg.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+    return v;
+}
+template <typename T> __device__ __forceinline__ T ld_act(const T *p) {
+    if constexpr (sizeof(T) == 4) {
+        const float v = ld_act_f32(reinterpret_cast<const float *>(p));
+        return *reinterpret_cast<const T *>(&v);
+    } else {
+        const unsigned short v = ld_act_u16(p);
+        return *reinterpret_cast<const T *>(&v);
+    }
+}
+
 // Dispatch a functor template over the three element types.
 #define XN_DISPATCH_DTYPE(dt, T, ...)                                                         \
     do {                                                                                      \
@@ -147,7 +186,7 @@ int launch_gemm_generic(xn_dtype dt, void *dst, const void *lhs, const void *rhs
 
 bool gemv_h16_single_chunk(size_t m, size_t k);
 int launch_gemv_h16(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k, size_t dst_rs,
-                    size_t lhs_rs, size_t rhs_cs, cudaStream_t st);
+                    size_t lhs_rs, size_t rhs_cs, const void *bias, cudaStream_t st);
 bool gemv_h16_batched_fits(size_t m, size_t n, size_t k, size_t batch);
 int launch_gemv_h16_batched(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k, size_t batch,
                             size_t lhs_bs, size_t rhs_bs, size_t dst_rs, size_t lhs_rs, size_t rhs_cs, cudaStream_t st);
@@ -161,6 +200,12 @@ int launch_gemv_f32x3(float *dst, const float *lhs, const float *rhs, size_t m, 
 int launch_gemv_dense(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k,
                       size_t lhs_b, size_t lhs_b_stride, size_t rhs_b_stride, size_t dst_rs, size_t lhs_rs, size_t rhs_cs,
                       cudaStream_t st);
+bool gemm_skinny_wanted(size_t m, size_t n, size_t k);
+int launch_skinny_fp8(void *y, const uint8_t *x_hi, const uint8_t *x_lo, const float *x_scale, const uint8_t *wq,
+                      const float *w_scale, size_t m, size_t n, size_t k, size_t ldy, cudaStream_t st);
+int launch_skinny_16bit(xn_dtype dt, void *dst, const void *lhs, const void *rhs, const void *bias, size_t m, size_t n, size_t k,
+                        size_t lda, size_t ldb, size_t ldd, size_t batch, size_t lhs_bs, size_t rhs_bs, size_t dst_bs, bool w_mn,
+                        cudaStream_t st);
 int launch_gemm_tn_16bit(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k,
                          size_t lda, size_t ldb, size_t ldd, size_t batch, size_t lhs_bs, size_t rhs_bs, cudaStream_t st,
                          int causal = 0, int causal_off = 0);

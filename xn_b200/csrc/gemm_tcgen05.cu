@@ -28,150 +28,12 @@
 //
 // Every mbarrier wait is bounded in time (wait.cuh); a wait that gives up reports it through the device's
 // host-visible status word and the CTA drains through its common exit (tensor memory is always released).
-#include <cuda.h>
-
-#include "common.cuh"
-#include "wait.cuh"
+#include "tc05.cuh"
 
 namespace xn {
 namespace {
 
-constexpr int BM = 128;        // rows of A per tile = TMEM lanes
-constexpr int BKB = 128;       // bytes of K per stage = one 128-byte swizzle atom
-constexpr int UMMA_KB = 32;    // bytes of K per tcgen05.mma (32 x 8-bit or 16 x 16-bit)
 constexpr int NTHREADS = 192;
-__device__ __forceinline__ unsigned smem_u32(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t *b, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *b, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
-}
-// Pull a tensor map (a kernel parameter) into the TMA unit's descriptor cache: the first copy that names it then
-// does not start with a fetch of the descriptor.
-__device__ __forceinline__ void prefetch_tmap(const CUtensorMap *m) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx_only(uint64_t *b, unsigned bytes) {  // no arrival
-    asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t *b) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(b)) : "memory");
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t *b, unsigned parity, const WaitCtx &w) {
-    return mbar_wait_bounded(smem_u32(b), parity, w);
-}
-
-__device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            smem_u32(dst)),
-        "l"(map), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-        : "memory");
-}
-__device__ __forceinline__ void tma_load_2d(void *dst, const CUtensorMap *map, int x, int y, uint64_t *bar) {
-    asm volatile(
-        "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-            smem_u32(dst)),
-        "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar))
-        : "memory");
-}
-
-// Shared-memory matrix descriptor: K-major tile, 128-byte swizzle, 8-row groups 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc(const void *tile) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_u32(tile) & 0x3FFFFu) >> 4);  // start address
-    d |= (uint64_t)0 << 16;                             // leading byte offset: unused for swizzled K-major
-    d |= (uint64_t)(1024 >> 4) << 32;                   // stride byte offset between 8-row groups
-    d |= (uint64_t)1 << 46;                             // descriptor version
-    d |= (uint64_t)2 << 61;                             // SWIZZLE_128B
-    return d;
-}
-
-// The same for an MN-major operand (the [K, N] right-hand side of a plain `matmul`, n contiguous): the tile is a
-// row of 64-column blocks, each block = BK k-rows of 128 bytes as TMA writes them with the 128-byte swizzle.
-// Within a block the 8-row groups along k are 1024 bytes apart (stride byte offset), the blocks along n
-// `block_bytes` apart (leading byte offset).
-__device__ __forceinline__ uint64_t smem_desc_mn(const void *tile, unsigned block_bytes) {
-    uint64_t d = 0;
-    d |= (uint64_t)((smem_u32(tile) & 0x3FFFFu) >> 4);
-    d |= (uint64_t)(block_bytes >> 4) << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-
-// Instruction descriptor: D = f32, A/B formats, both K-major, N >> 3 at bit 17, M >> 4 at bit 24.
-__host__ __device__ constexpr uint32_t instr_desc(int a_fmt, int b_fmt, int n) {
-    return (1u << 4) | ((uint32_t)a_fmt << 7) | ((uint32_t)b_fmt << 10) | ((uint32_t)(n >> 3) << 17) |
-           ((uint32_t)(BM >> 4) << 24);
-}
-
-template <bool F8>
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-    if (F8)
-        asm volatile(
-            "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-            "tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-            "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-            : "memory");
-    else
-        asm volatile(
-            "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-            "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-            : "memory");
-}
-__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-        "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc)
-        : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t *bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
-        "%29,%30,%31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// issue only: the caller waits once for all its loads
-__device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t *v) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-        "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,"
-        "%29,%30,%31}, [%32];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-          "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-          "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-          "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-        : "r"(taddr));
-}
-
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,"
-        "%30,%31,%32};" ::"r"(taddr),
-        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
-        "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
-        "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
-    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-}
 
 // Tile order within one batch entry.  Tiles that run at the same time (148 consecutive indices) should share as
 // many operand panels as possible, or every wave re-reads both operands from HBM (at 8192^3 the plain m-fastest
@@ -262,7 +124,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmArgs &args, uint32_t tme
     }
     const int row = m_row0 + q * 32 + lane;
     float xs = 1.0f;
-    if (F8 && row < args.M) xs = __ldg(args.x_scale + row);
+    if (F8 && row < args.M) xs = ld_act_f32(args.x_scale + row);
     float rb = 0.0f;
     if (!F8 && args.row_bias && row < args.M)
         rb = KIND == 2 ? __half2float(reinterpret_cast<const __half *>(args.row_bias)[row])
@@ -421,7 +283,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
     __shared__ __align__(8) uint64_t full[NSTAGE], empty[NSTAGE], tmem_full[2], tmem_empty[2];
     __shared__ uint32_t tmem_slot;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_id(), lane = threadIdx.x & 31;
     const int BMT = (NA == 2 && args.rows2) ? 2 * BM : BM;  // rows of A per tile
     const int num_m = (args.M + BMT - 1) / BMT, num_n = (args.N + BN - 1) / BN;
     const int tiles_per_batch = num_m * num_n;
@@ -454,7 +316,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
 
     if (warp == 0) {
         // ---------------- producer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             int it = 0;  // running k-block count across tiles: stage = it % NSTAGE
             bool ok = true;
             for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -491,7 +353,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
-        if (lane == 0) {
+        if (elect_one()) {
             int it = 0, vt = 0;   // vt: accumulator hand-overs to the epilogue so far (one per tile, or per k chunk)
             bool ok = true;
             for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -516,15 +378,15 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
                     if (!mbar_wait(&full[s], ph, args.wait)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     unsigned char *st = smem + (size_t)s * STAGE_BYTES;
-                    const uint64_t da0 = smem_desc(st), da1 = smem_desc(st + A_BYTES);
+                    const uint32_t da0 = smem_desc(st), da1 = smem_desc(st + A_BYTES);
                     const bool bmn = ELEM == 2 && args.b_mn;
-                    const uint64_t db = bmn ? smem_desc_mn(st + NA * A_BYTES, 64 * BKB) : smem_desc(st + NA * A_BYTES);
+                    const uint32_t db = bmn ? smem_desc_mn(st + NA * A_BYTES, 64 * BKB) : smem_desc(st + NA * A_BYTES);
                     const uint32_t idesc = bmn ? (IDESC | (1u << 16)) : IDESC;   // bit 16: B is MN-major
                     // k advance per MMA: 32 bytes inside the swizzled row (K-major), 16 k-rows of 128 bytes (MN-major)
-                    const uint64_t badv = bmn ? (uint64_t)((UMMA_KB / ELEM) * 128 >> 4) : (uint64_t)(UMMA_KB >> 4);
+                    const uint32_t badv = bmn ? (uint32_t)((UMMA_KB / ELEM) * 128 >> 4) : (uint32_t)(UMMA_KB >> 4);
 #pragma unroll
                     for (int ks = 0; ks < BKB / UMMA_KB; ++ks) {
-                        const uint64_t adv = (uint64_t)(ks * UMMA_KB >> 4);
+                        const uint32_t adv = (uint32_t)(ks * UMMA_KB >> 4);
                         if constexpr (KIND == 3) {
                             umma_tf32(d_tmem, da0 + adv, db + adv, IDESC, kb > kb0 || ks != 0);
                         } else {
@@ -669,340 +531,6 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
 }
 
 // ---------------------------------------------------------------------------------------------
-// Skinny form for 8 < M <= 64 (weights >> activations, HBM-bound): the operands swap roles.  The
-// 128 TMEM lanes carry 128 output channels (a 16 KB weight tile per 128-byte k stage) and the MMA's N
-// dimension carries the M activation rows (one or two e4m3 pieces of MB rows each), so almost all
-// bytes in flight are weight bytes and a deep ring (up to 8 stages) keeps ~100 KB of them in flight
-// per SM.  D[n, m] is written transposed: lane = output channel, column = activation row.
-// ---------------------------------------------------------------------------------------------
-struct SkinnyArgs {
-    void *y;     // [M, ldy] bf16 (fp8 and bf16 operands) or f16
-    int ldy;
-    const float *x_scale, *w_scale;  // fp8 operands only
-    float *partials;     // scratch: [2 * grid][MB][128] f32 partial accumulators of split tiles
-    unsigned *counters;  // scratch: [tiles] arrival counts; zero between launches
-    int M, N, K;
-    int MB;      // MMA N dimension: M rounded up to 16
-    int nstage;
-    int np;      // pieces (1 or 2)
-    int uq, ur;  // stage units per CTA: total / grid and total % grid
-    int w_static;  // the weights are a model parameter: they may be fetched before the dependency wait
-    WaitCtx wait;  // bound and status word of the kernel's mbarrier waits
-};
-
-// Work is cut at k-stage granularity ("stream-K"): total = tiles * num_kb stage units, CTA c owns the
-// contiguous unit range [c*total/G, (c+1)*total/G), i.e. a run of segments (tile, kb0..kb1).  A tile
-// that is covered by several CTAs is finished by whichever of them arrives last:
-// every contributor stores its f32 partial to scratch, and the finisher adds all partials in k order
-// -- a fixed order, so the result does not depend on which CTA happens to be last.
-// (32-bit arithmetic only: a 64-bit division is ~100 dependent instructions, and the epilogue warps sit on
-// the critical path at the end of the kernel.)  uq = total / G, ur = total % G come from the host: the first ur
-// CTAs own uq + 1 units, the others uq.
-__device__ __forceinline__ int unit_begin(int c, int uq, int ur) { return c * uq + min(c, ur); }
-__device__ __forceinline__ int unit_owner(int u, int uq, int ur) {  // the CTA whose range holds unit u
-    const int big = ur * (uq + 1);
-    return u < big ? (int)((unsigned)u / (unsigned)(uq + 1)) : ur + (int)((unsigned)(u - big) / (unsigned)uq);
-}
-
-// The finisher's sum over a split tile's contributors.  The four epilogue warps of the CTA that arrived last share
-// the tile's rows (warp w takes rows w, w + 4, ...); a lane owns four consecutive channels, so one 128-bit load per
-// (row, contributor) and one 8-byte store per row replace four scalar ones -- the reduction is the tail of the
-// kernel and was bound by its own instruction count on one warp per scheduler.  RB rows x NC contributors are in
-// flight per round; the additions run in contributor (= k) order whatever the arrival order was.
-template <int KIND, int RB, int NC>
-__device__ __forceinline__ void skinny_reduce(const SkinnyArgs &args, const float *s_xs, int tile, int w, int lane, int c_first,
-                                              int c_last, int t0, int uq, int ur, size_t slot_elems) {
-    constexpr bool F8 = KIND == 0;
-    const int ch0 = tile * BM + 4 * lane;  // first of this lane's four channels
-    float ws[4] = {1.0f, 1.0f, 1.0f, 1.0f};
-    if (F8) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) ws[i] = ch0 + i < args.N ? __ldg(args.w_scale + ch0 + i) : 0.0f;
-    }
-    const bool vec_store = ch0 + 4 <= args.N && (args.ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(args.y) & 7) == 0;
-    for (int m0 = w; m0 < args.M; m0 += 4 * RB) {
-        float4 sum[RB];
-#pragma unroll
-        for (int j = 0; j < RB; ++j) sum[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int cc0 = c_first; cc0 <= c_last; cc0 += NC) {
-            float4 tv[NC][RB];
-#pragma unroll
-            for (int d = 0; d < NC; ++d) {
-                const int cc = cc0 + d;
-                const bool on = cc <= c_last;
-                const int slot = on ? 2 * cc + (unit_begin(cc, uq, ur) >= t0 ? 0 : 1) : 0;
-                const float *src = args.partials + (size_t)slot * slot_elems + 4 * lane;
-#pragma unroll
-                for (int j = 0; j < RB; ++j) {
-                    const int row = m0 + 4 * j;
-                    tv[d][j] = (on && row < args.M) ? __ldcg(reinterpret_cast<const float4 *>(src + (size_t)row * BM))
-                                                    : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            }
-#pragma unroll
-            for (int d = 0; d < NC; ++d)
-#pragma unroll
-                for (int j = 0; j < RB; ++j) {
-                    sum[j].x += tv[d][j].x; sum[j].y += tv[d][j].y; sum[j].z += tv[d][j].z; sum[j].w += tv[d][j].w;
-                }
-        }
-#pragma unroll
-        for (int j = 0; j < RB; ++j) {
-            const int row = m0 + 4 * j;
-            if (row >= args.M) continue;
-            const float xs = F8 ? s_xs[row] : 1.0f;
-            const float val[4] = {F8 ? ws[0] * (xs * sum[j].x) : sum[j].x, F8 ? ws[1] * (xs * sum[j].y) : sum[j].y,
-                                  F8 ? ws[2] * (xs * sum[j].z) : sum[j].z, F8 ? ws[3] * (xs * sum[j].w) : sum[j].w};
-            if (KIND == 2) {
-                __half *dst = reinterpret_cast<__half *>(args.y) + (size_t)row * args.ldy + ch0;
-                if (vec_store) {
-                    const __half2 lo = __floats2half2_rn(val[0], val[1]), hi = __floats2half2_rn(val[2], val[3]);
-                    *reinterpret_cast<uint2 *>(dst) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
-                } else {
-                    for (int i = 0; i < 4; ++i)
-                        if (ch0 + i < args.N) dst[i] = __float2half_rn(val[i]);
-                }
-            } else {
-                __nv_bfloat16 *dst = reinterpret_cast<__nv_bfloat16 *>(args.y) + (size_t)row * args.ldy + ch0;
-                if (vec_store) {
-                    const __nv_bfloat162 lo = __floats2bfloat162_rn(val[0], val[1]), hi = __floats2bfloat162_rn(val[2], val[3]);
-                    *reinterpret_cast<uint2 *>(dst) = make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
-                } else {
-                    for (int i = 0; i < 4; ++i)
-                        if (ch0 + i < args.N) dst[i] = __float2bfloat16_rn(val[i]);
-                }
-            }
-        }
-    }
-}
-
-// KIND: 0 = fp8 pieces -> bf16 out (scaled), 1 = bf16 -> bf16, 2 = f16 -> f16 (one piece, no scales)
-template <int KIND>
-__global__ void __launch_bounds__(NTHREADS, 1)
-gemm_tcgen05_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x0,
-                           const __grid_constant__ CUtensorMap map_x1, const SkinnyArgs args) {
-    constexpr int W_BYTES = BM * BKB;
-    const int X_BYTES = args.MB * BKB;
-    const int STAGE_BYTES = W_BYTES + args.np * X_BYTES;
-    const int NSTAGE = args.nstage;
-    // One MMA per k step covers both pieces: they sit back to back in the stage, so they form one
-    // K-major operand of np * MB rows; D columns [0, MB) are the hi products, [MB, 2 MB) the lo products
-    // (an MMA instruction costs about 130 cycles here however small N is: fewer, wider MMAs).
-    const int NB = args.np * args.MB;  // MMA N dimension = TMEM columns of one accumulator buffer
-    constexpr bool F8 = KIND == 0;
-    const uint32_t IDESC = KIND == 1 ? instr_desc(1, 1, NB) : instr_desc(0, 0, NB);
-    const int TMEM_COLS = 2 * NB <= 32 ? 32 : (2 * NB <= 64 ? 64 : (2 * NB <= 128 ? 128 : (2 * NB <= 256 ? 256 : 512)));
-
-    extern __shared__ unsigned char smem_raw[];
-    unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t full[8], empty[8], tmem_full[2], tmem_empty[2];
-    __shared__ uint32_t tmem_slot;
-    __shared__ float s_xs[64];  // x_scale of the (at most 64) activation rows
-    __shared__ int s_ok[2][4];  // per segment parity: has each epilogue warp seen its accumulator?
-    __shared__ int s_last;      // this CTA arrived last at the split tile of the current segment
-
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int num_kb = (args.K + (KIND == 0 ? BKB : BKB / 2) - 1) / (KIND == 0 ? BKB : BKB / 2);
-    const int uq = args.uq, ur = args.ur;
-    const int u0 = unit_begin(blockIdx.x, uq, ur), u1 = unit_begin(blockIdx.x + 1, uq, ur);
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-
-    if (threadIdx.x == 0) {
-        prefetch_tmap(&map_w);
-        prefetch_tmap(&map_x0);
-        if (args.np == 2) prefetch_tmap(&map_x1);
-        for (int s = 0; s < NSTAGE; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(&tmem_full[a], 1); mbar_init(&tmem_empty[a], 4); }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
-                     "r"(TMEM_COLS)
-                     : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = tmem_slot;
-
-    // Programmatic dependent launch.  The kernel is small enough (shared memory, registers, tensor-memory
-    // columns) for two of them to share an SM, so the next launch's CTAs set up, allocate and -- since
-    // weights do not depend on the previous kernel -- fetch the weight halves of their first ring-full while
-    // this one is still running.  Activations, scales, the output and the split-tile scratch belong to the
-    // stream order: the producer waits before its first activation load, the epilogue warps before their
-    // first global access; the MMA warp only reads shared memory.
-    if (warp == 0) {
-        if (lane == 0) {
-            constexpr int BK = F8 ? BKB : BKB / 2;  // k elements per stage
-            const int pre = min(NSTAGE, u1 - u0);
-            if (!args.w_static) asm volatile("griddepcontrol.wait;" ::: "memory");  // the previous kernel may have written w
-            for (int it = 0; it < pre; ++it) {
-                const int u = u0 + it;
-                const int tile = (int)((unsigned)u / (unsigned)num_kb), kb = u - tile * num_kb;
-                mbar_expect_tx_only(&full[it], (unsigned)W_BYTES);
-                tma_load_2d(smem + (size_t)it * STAGE_BYTES, &map_w, kb * BK, tile * BM, &full[it]);
-            }
-            asm volatile("griddepcontrol.wait;" ::: "memory");
-            int it = 0;
-            bool ok = true;
-            for (int u = u0; u < u1 && ok;) {
-                const int tile = (int)((unsigned)u / (unsigned)num_kb), kb0 = u - tile * num_kb;
-                const int kb1 = min(num_kb, kb0 + (u1 - u));
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int s = it % NSTAGE;
-                    const unsigned ph = (unsigned)(it / NSTAGE) & 1u;
-                    unsigned char *st = smem + (size_t)s * STAGE_BYTES;
-                    if (it < pre) {  // the weights of this stage are already on their way
-                        mbar_expect_tx(&full[s], (unsigned)(args.np * X_BYTES));
-                    } else {
-                        if (!mbar_wait(&empty[s], ph ^ 1u, args.wait)) { ok = false; break; }
-                        mbar_expect_tx(&full[s], STAGE_BYTES);
-                        tma_load_2d(st, &map_w, kb * BK, tile * BM, &full[s]);
-                    }
-                    tma_load_2d(st + W_BYTES, &map_x0, kb * BK, 0, &full[s]);
-                    if (args.np == 2) tma_load_2d(st + W_BYTES + X_BYTES, &map_x1, kb * BK, 0, &full[s]);
-                }
-                u += kb1 - kb0;
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            int it = 0, t_local = 0;
-            bool ok = true;
-            for (int u = u0; u < u1 && ok; ++t_local) {
-                const int kb0 = u - (int)((unsigned)u / (unsigned)num_kb) * num_kb;
-                const int kb1 = min(num_kb, kb0 + (u1 - u));
-                const int acc = t_local & 1;
-                const unsigned acc_ph = (unsigned)(t_local >> 1) & 1u;
-                if (!mbar_wait(&tmem_empty[acc], acc_ph ^ 1u, args.wait)) { ok = false; break; }
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t d_tmem = tmem_base + (uint32_t)(acc * NB);
-                for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int s = it % NSTAGE;
-                    const unsigned ph = (unsigned)(it / NSTAGE) & 1u;
-                    if (!mbar_wait(&full[s], ph, args.wait)) { ok = false; break; }
-                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    unsigned char *st = smem + (size_t)s * STAGE_BYTES;
-                    const uint64_t dw = smem_desc(st), dx = smem_desc(st + W_BYTES);
-#pragma unroll
-                    for (int ks = 0; ks < BKB / UMMA_KB; ++ks) {
-                        const uint64_t adv = (uint64_t)(ks * UMMA_KB >> 4);
-                        umma<F8>(d_tmem, dw + adv, dx + adv, IDESC, (kb > kb0) || ks != 0);
-                    }
-                    umma_commit(&empty[s]);
-                }
-                if (ok) umma_commit(&tmem_full[acc]);
-                u += kb1 - kb0;
-            }
-        }
-    } else {
-        const int q = warp & 3;
-        int t_local = 0;
-        bool ok = true;
-        const size_t slot_elems = (size_t)args.MB * BM;
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-        if (F8 && warp == 2) {
-            s_xs[lane] = lane < args.M ? __ldg(args.x_scale + lane) : 0.0f;
-            s_xs[lane + 32] = lane + 32 < args.M ? __ldg(args.x_scale + lane + 32) : 0.0f;
-        }
-        asm volatile("bar.sync 1, 128;" ::: "memory");  // the four epilogue warps
-        for (int u = u0; u < u1 && ok; ++t_local) {
-            const int tile = (int)((unsigned)u / (unsigned)num_kb), kb0 = u - tile * num_kb;
-            const int kb1 = min(num_kb, kb0 + (u1 - u));
-            const bool whole = kb0 == 0 && kb1 == num_kb;
-            const int acc = t_local & 1;
-            const unsigned acc_ph = (unsigned)(t_local >> 1) & 1u;
-            // The four warps act together below (named barrier 1): a warp whose wait ran out still takes part in this
-            // segment's barrier, and all four leave the loop together.
-            const bool got = mbar_wait(&tmem_full[acc], acc_ph, args.wait);
-            if (lane == 0) s_ok[t_local & 1][q] = got ? 1 : 0;
-            asm volatile("bar.sync 1, 128;" ::: "memory");
-            if (!(s_ok[t_local & 1][0] && s_ok[t_local & 1][1] && s_ok[t_local & 1][2] && s_ok[t_local & 1][3])) { ok = false; break; }
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const int ch = tile * BM + q * 32 + lane;  // output channel of this lane
-            const float ws = !F8 ? 1.0f : (ch < args.N ? __ldg(args.w_scale + ch) : 0.0f);
-            // a split tile's segment is this CTA's first one iff its range starts inside that tile
-            const int my_slot = 2 * blockIdx.x + ((u == u0) ? 0 : 1);
-            float *mine = args.partials + (size_t)my_slot * slot_elems + q * 32 + lane;
-#pragma unroll 1
-            for (int c = 0; c < args.MB; c += 16) {
-                uint32_t v[16];
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                      "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                    : "r"(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * NB + c)));
-                if (args.np == 2) {
-                    uint32_t w[16];
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-                        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]),
-                          "=r"(w[8]), "=r"(w[9]), "=r"(w[10]), "=r"(w[11]), "=r"(w[12]), "=r"(w[13]), "=r"(w[14]), "=r"(w[15])
-                        : "r"(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * NB + args.MB + c)));
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + __uint_as_float(w[j]));
-                } else {
-                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                }
-                if (whole) {
-                    if (ch < args.N) {
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const int mrow = c + j;
-                            if (mrow < args.M) {  // 32 lanes = 32 consecutive channels of one activation row
-                                const float val = F8 ? ws * (s_xs[mrow] * __uint_as_float(v[j])) : __uint_as_float(v[j]);
-                                if (KIND == 2) reinterpret_cast<__half *>(args.y)[(size_t)mrow * args.ldy + ch] = __float2half_rn(val);
-                                else reinterpret_cast<__nv_bfloat16 *>(args.y)[(size_t)mrow * args.ldy + ch] = __float2bfloat16_rn(val);
-                            }
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) mine[(size_t)(c + j) * BM] = __uint_as_float(v[j]);
-                }
-            }
-            // the accumulator buffer can be reused as soon as it has been read
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty[acc]);
-
-            if (!whole) {
-                // contributors of this tile: the CTAs whose unit ranges intersect [tile*num_kb, (tile+1)*num_kb)
-                const int t0 = tile * num_kb, t1 = t0 + num_kb;
-                const int c_first = unit_owner(t0, uq, ur), c_last = unit_owner(t1 - 1, uq, ur);
-                const unsigned ncontrib = (unsigned)(c_last - c_first + 1);
-                __threadfence();  // this warp's quarter of the partial is visible before the CTA is counted
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (warp == 2 && lane == 0) s_last = atomicAdd(args.counters + tile, 1u) == ncontrib - 1 ? 1 : 0;
-                asm volatile("bar.sync 1, 128;" ::: "memory");
-                if (s_last) {  // last arriver: reduce in k order and store
-                    __threadfence();
-                    if (warp == 2 && lane == 0) args.counters[tile] = 0;  // ready for the next launch
-                    // Every round of loads is an L2 round trip on the critical path at the end of the kernel: 16
-                    // 128-bit loads per lane are in flight per round (8 rows x 2 contributors when a tile has at most
-                    // two, 4 rows x 4 otherwise).
-                    if (c_last - c_first < 2)
-                        skinny_reduce<KIND, 8, 2>(args, s_xs, tile, warp - 2, lane, c_first, c_last, t0, uq, ur, slot_elems);
-                    else
-                        skinny_reduce<KIND, 4, 4>(args, s_xs, tile, warp - 2, lane, c_first, c_last, t0, uq, ur, slot_elems);
-                }
-            }
-            u += kb1 - kb0;
-        }
-    }
-
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (warp == 1) {
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
-    }
-}
-
-// ---------------------------------------------------------------------------------------------
 // Block-quantized integer weights with many activation rows: kind::i8 MMAs (s8 x s8 -> s32, exact) with one
 // hand-over per 32-element block.  The operands swap roles as in the skinny form: the 128 TMEM lanes carry 128
 // output channels (row-major int8 weights, unpacked from the q4 / q8 tiles by a pre-pass), the MMA's N dimension
@@ -1027,11 +555,11 @@ struct QGemmArgs {
 __host__ __device__ constexpr uint32_t instr_desc_i8(int n) {  // D = s32, A and B signed 8-bit, both K-major
     return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 }
-__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t a_desc, uint64_t b_desc, uint32_t idesc) {  // D = A * B
+__device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint32_t a_desc, uint32_t b_desc, uint32_t idesc) {  // D = A * B
     asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, 0, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-        "l"(a_desc), "l"(b_desc), "r"(idesc)
+        "{\n.reg .pred p;\n.reg .b64 a, b;\nmov.b64 a, {%1, %4};\nmov.b64 b, {%2, %4};\nsetp.ne.b32 p, 0, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], a, b, %3, p;\n}" ::"r"(tmem_d),
+        "r"(a_desc), "r"(b_desc), "r"(idesc), "n"(DESC_HI)
         : "memory");
 }
 // An int32 block sum plus 0x4B400000, read as a float, is 1.5 * 2^23 + sum exactly (|sum| <= 32 * 127 * 127 < 2^22):
@@ -1055,7 +583,7 @@ gemm_q8_block_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     __shared__ __align__(8) uint64_t full[NSTAGE], empty[NSTAGE], acc_full[NACC], acc_empty[NACC];
     __shared__ uint32_t tmem_slot;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_id(), lane = threadIdx.x & 31;
     const int num_w = (args.NPAD + BM - 1) / BM, num_x = (args.MA + BN - 1) / BN;
     const int num_tiles = num_w * num_x;
     const int num_kb = args.K / BKB;
@@ -1082,7 +610,7 @@ gemm_q8_block_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             int it = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -1098,7 +626,7 @@ gemm_q8_block_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             int it = 0;
             unsigned vt = 0;  // hand-overs so far
             bool ok = true;
@@ -1108,12 +636,12 @@ gemm_q8_block_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                     if (!mbar_wait(&full[s], (unsigned)(it / NSTAGE) & 1u, args.wait)) { ok = false; break; }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     unsigned char *st = smem + (size_t)s * STAGE_BYTES;
-                    const uint64_t dw = smem_desc(st), dx = smem_desc(st + W_BYTES);
+                    const uint32_t dw = smem_desc(st), dx = smem_desc(st + W_BYTES);
                     for (int ks = 0; ks < BPS; ++ks, ++vt) {
                         const unsigned a = vt % NACC;
                         if (!mbar_wait(&acc_empty[a], ((vt / NACC) & 1u) ^ 1u, args.wait)) { ok = false; break; }
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        const uint64_t adv = (uint64_t)(ks * UMMA_KB >> 4);
+                        const uint32_t adv = (uint32_t)(ks * UMMA_KB >> 4);
                         umma_i8(tmem_base + a * BN, dw + adv, dx + adv, IDESC);
                         umma_commit(&acc_full[a]);
                     }
@@ -1183,8 +711,8 @@ gemm_q8_block_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_con
                     float a0, a1;
                     asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(acc2[i / 2]));
                     const int row = x_blk * BN + half * HALF + i;  // 32 lanes = 32 consecutive channels of one activation row
-                    if (row < args.MA) args.y[(size_t)row * args.ldy + ch] = __ldg(args.x_scale + row) * a0;
-                    if (row + 1 < args.MA) args.y[(size_t)(row + 1) * args.ldy + ch] = __ldg(args.x_scale + row + 1) * a1;
+                    if (row < args.MA) args.y[(size_t)row * args.ldy + ch] = ld_act_f32(args.x_scale + row) * a0;
+                    if (row + 1 < args.MA) args.y[(size_t)(row + 1) * args.ldy + ch] = ld_act_f32(args.x_scale + row + 1) * a1;
                 }
             }
         }
@@ -1236,11 +764,11 @@ __device__ __forceinline__ float ex2_approx(float x) {
 }
 
 // D += A * B with the A operand in tensor memory (lane = row, two 16-bit elements per column, 8 columns per MMA)
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t b_desc, uint32_t idesc, uint32_t acc) {
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint32_t b_desc, uint32_t idesc, uint32_t acc) {
     asm volatile(
-        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(b_desc), "r"(idesc), "r"(acc)
+        "{\n.reg .pred p;\n.reg .b64 b;\nmov.b64 b, {%2, %5};\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b, %3, p;\n}" ::"r"(tmem_d),
+        "r"(tmem_a), "r"(b_desc), "r"(idesc), "r"(acc), "n"(DESC_HI)
         : "memory");
 }
 
@@ -1258,7 +786,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     __shared__ uint32_t tmem_slot;
     __shared__ float red_m[2][128], red_l[2][128];
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_id(), lane = threadIdx.x & 31;
     // The kernel is persistent: CTA c works on items c, c + grid, ... of the list of (query block, head) pairs ordered
     // by falling work (the last query block of every head first), so that every CTA gets the same share within a block
     // or two, and the set-up, the first loads and the first scores of an item overlap the tail of the previous one.
@@ -1307,7 +835,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             unsigned g = 0, n_item = 0;  // key blocks and items so far
             for (int item = first_item(0); item < nitems && ok; item = first_item(++n_item)) {
@@ -1336,7 +864,7 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (elect_one()) {
             bool ok = true;
             unsigned gs = 0, gp = 0, n_item = 0;  // scores issued, products issued, items so far
             // S[gs & 1] = Q K^T for the next key block of the K ring
@@ -1347,10 +875,10 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const uint64_t da = smem_desc(sQ + h * ATT_TILE), db = smem_desc(sK + (2 * b + h) * ATT_TILE);
+                    const uint32_t da = smem_desc(sQ + h * ATT_TILE), db = smem_desc(sK + (2 * b + h) * ATT_TILE);
 #pragma unroll
                     for (int ks = 0; ks < BKB / UMMA_KB; ++ks) {
-                        const uint64_t adv = (uint64_t)(ks * UMMA_KB >> 4);
+                        const uint32_t adv = (uint32_t)(ks * UMMA_KB >> 4);
                         umma<false>(tmem_base + b * 128, da + adv, db + adv, IDESC, (h | ks) != 0);
                     }
                 }
@@ -1379,10 +907,10 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                     for (int kh = 0; kh < 2; ++kh) {  // stream kh: O_kh += P[:, keys of half kh] V[keys of half kh]
-                        const uint64_t db = smem_desc_mn(sV + (2 * b + kh) * ATT_TILE, 64 * BKB);
+                        const uint32_t db = smem_desc_mn(sV + (2 * b + kh) * ATT_TILE, 64 * BKB);
 #pragma unroll
                         for (int ks = 0; ks < BKB / UMMA_KB; ++ks) {
-                            const uint64_t badv = (uint64_t)((UMMA_KB / 2) * 128 >> 4);  // 16 key rows of 128 bytes per MMA
+                            const uint32_t badv = (uint32_t)((UMMA_KB / 2) * 128 >> 4);  // 16 key rows of 128 bytes per MMA
                             // P of stream kh sits in the first 32 columns of the stream's half of S[b]: 8 columns per MMA
                             umma_ts(tmem_o + kh * 128, tmem_base + b * 128 + kh * 64 + ks * 8, db + ks * badv, IDESC | (1u << 16),
                                     (j | ks) != 0);
@@ -1537,84 +1065,6 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 }
 
 // ---- host side ----
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
-                                  const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
-                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_fn() {
-    static EncodeTiledFn fn = [] {
-        void *p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            p = nullptr;
-        return (EncodeTiledFn)p;
-    }();
-    return fn;
-}
-
-// 2-D row-major [rows, k] tensor with `elem` bytes per element and a row pitch of ld elements;
-// box = 128 bytes of k by box_rows rows, 128-byte swizzle, out-of-range reads give zeros.
-// 3-D form of the same map: `batch` matrices `batch_stride` elements apart (box covers one of them).
-// Dimensions are ordered by increasing stride: when the batch stride is smaller than the row pitch (a
-// transposed view such as [groups, rows, k] over storage [rows, groups, k]) the map is (k, batch, rows) and
-// *batch_inner is set; the shared-memory image of a box is the same either way.
-int make_map3(CUtensorMap *map, const void *base, int elem, size_t rows, size_t k, size_t ld, int box_rows,
-              size_t batch, size_t batch_stride, int *batch_inner) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail(XN_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-    if (batch <= 1) { batch = 1; batch_stride = rows * ld; }
-    const bool inner = batch_stride < ld;
-    *batch_inner = inner ? 1 : 0;
-    cuuint64_t dims[3] = {(cuuint64_t)k, (cuuint64_t)(inner ? batch : rows), (cuuint64_t)(inner ? rows : batch)};
-    cuuint64_t strides[2] = {(cuuint64_t)(inner ? batch_stride : ld) * elem, (cuuint64_t)(inner ? ld : batch_stride) * elem};
-    cuuint32_t box[3] = {(cuuint32_t)(BKB / elem), (cuuint32_t)(inner ? 1 : box_rows), (cuuint32_t)(inner ? box_rows : 1)};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUtensorMapDataType dt = elem == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
-                                       : (elem == 4 ? CU_TENSOR_MAP_DATA_TYPE_UINT32 : CU_TENSOR_MAP_DATA_TYPE_UINT16);
-    CUresult r = fn(map, dt, 3, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(XN_ERR_CUDA, "cuTensorMapEncodeTiled (3-D) failed with code %d", (int)r);
-    return XN_OK;
-}
-
-int make_map(CUtensorMap *map, const void *base, int elem, size_t rows, size_t k, size_t ld, int box_rows) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail(XN_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-    cuuint64_t dims[2] = {(cuuint64_t)k, (cuuint64_t)rows};
-    cuuint64_t strides[1] = {(cuuint64_t)ld * elem};
-    cuuint32_t box[2] = {(cuuint32_t)(BKB / elem), (cuuint32_t)box_rows};
-    cuuint32_t estr[2] = {1, 1};
-    CUtensorMapDataType dt = elem == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_UINT16;
-    CUresult r = fn(map, dt, 2, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(XN_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", (int)r);
-    return XN_OK;
-}
-
-// [K, N] operand with n contiguous, k-rows `ld` elements apart, `batch` matrices batch_stride elements apart:
-// dimensions (n, k, batch), box 64 n x 64 k (128-byte rows, 128-byte swizzle).  16-bit elements only.
-// As in make_map3 the dimensions are ordered by increasing stride: when the matrices interleave (batch stride
-// smaller than the k-row pitch, e.g. the per-head value slices of a fused qkv projection) the map is (n, batch, k)
-// and *batch_inner is set.
-int make_map_mn(CUtensorMap *map, const void *base, size_t n, size_t k, size_t ld, size_t batch, size_t batch_stride,
-                int *batch_inner) {
-    EncodeTiledFn fn = encode_fn();
-    if (!fn) return fail(XN_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-    if (batch <= 1) { batch = 1; batch_stride = k * ld; }
-    const bool inner = batch_stride < ld;
-    *batch_inner = inner ? 1 : 0;
-    cuuint64_t dims[3] = {(cuuint64_t)n, (cuuint64_t)(inner ? batch : k), (cuuint64_t)(inner ? k : batch)};
-    cuuint64_t strides[2] = {(cuuint64_t)(inner ? batch_stride : ld) * 2, (cuuint64_t)(inner ? ld : batch_stride) * 2};
-    cuuint32_t box[3] = {64, (cuuint32_t)(inner ? 1 : BKB / 2), (cuuint32_t)(inner ? BKB / 2 : 1)};
-    cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void *>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) return fail(XN_ERR_CUDA, "cuTensorMapEncodeTiled (n-contiguous operand) failed with code %d", (int)r);
-    return XN_OK;
-}
-
 // Second half of a split-k product: y = epilogue(sum over the k chunks of the f32 tile records the tiled kernel left
 // in `rec`), the chunks added in k order.  A thread owns one row of a tile and one group of 4 columns; a CTA of 256
 // threads covers the tile's 128 rows x 2 column groups, so every record read is 512 contiguous bytes per warp.
@@ -1645,7 +1095,7 @@ splitk_reduce_kernel(void *__restrict__ y, int ldy, const float *__restrict__ re
     }
     float val[4] = {sum.x, sum.y, sum.z, sum.w};
     if (F8) {
-        const float xs = __ldg(x_scale + row);
+        const float xs = ld_act_f32(x_scale + row);
 #pragma unroll
         for (int e = 0; e < 4; ++e) val[e] = (col + e < N ? __ldg(w_scale + col + e) : 0.0f) * (xs * val[e]);
     }
@@ -1854,85 +1304,6 @@ int launch_kind(const void *a0, const void *a1, const void *b, size_t lda, size_
 
 }  // namespace
 
-// Skinny path, m <= 64.  KIND 0: e4m3 pieces x0 (hi) and optional x1 (lo) with scales; KIND 1 / 2: bf16 / f16
-// operands (x1, scales unused).  Strides in elements.
-template <int KIND>
-int launch_skinny(void *y, size_t ldy, const void *x0, const void *x1, size_t ldx, const float *x_scale, const void *w,
-                  size_t ldw, const float *w_scale, size_t m, size_t n, size_t k, cudaStream_t st) {
-    constexpr int ELEM = KIND == 0 ? 1 : 2;
-    constexpr int BK = BKB / ELEM;  // k elements per stage
-    SkinnyArgs a{};
-    a.y = y; a.ldy = (int)ldy; a.x_scale = x_scale; a.w_scale = w_scale;
-    a.M = (int)m; a.N = (int)n; a.K = (int)k;
-    a.MB = (int)((m + 15) / 16 * 16);
-    a.np = x1 ? 2 : 1;
-    const int stage = BM * BKB + a.np * a.MB * BKB;
-    // a ring of about 100 KB: two CTAs (this launch's and the next one's, see the kernel) fit an SM, and the
-    // kernel is not bound by bytes in flight (3 to 8 stages measured the same)
-    static const int ring_kb = [] { const char *e = getenv("XN_SKINNY_RING_KB"); return e ? atoi(e) : 100; }();
-    a.nstage = (ring_kb * 1024) / stage > 8 ? 8 : (ring_kb * 1024) / stage;
-    if (a.nstage < 2) a.nstage = 2;
-    const int tiles = (int)((n + BM - 1) / BM);
-    const int num_kb = (int)((k + BK - 1) / BK);
-    const int sms = sm_count();
-    const long long total = (long long)tiles * num_kb;
-    // at least 4 k stages per CTA, so that a split never degenerates into single-stage crumbs
-    long long grid = total / 4 < 1 ? 1 : total / 4;
-    if (grid > sms) grid = sms;
-    // Whole tiles (no fix-up pass) only when they fill at least 90 % of the machine; otherwise split at
-    // k-stage granularity so that every SM streams its share of the weights and issues its share of the MMAs
-    // (an MMA costs ~130 cycles whatever its N, so the MMA count per CTA is what bounds a skinny problem).
-    if (tiles <= sms && tiles * 100 >= sms * 90) grid = tiles;
-    // Fewer tiles than SMs: S = SMs / tiles CTAs per tile, cut at the same k positions in every tile, when that
-    // still occupies 60 % of the machine.  Every tile then has exactly S contributors (S = 1: none) instead of the
-    // S + 1 or S + 2 ragged ones of the even split over all SMs, and the last arriver's reduction -- the tail of
-    // the kernel -- gets shorter by more than the k loop gets longer.  Measured (fp8, 32 / 64 rows): N = 4096,
-    // k = 4096 on 128 CTAs 12.6 -> 11.2 / 18.1 -> 15.4 us; k = 11264 17.7 -> 17.0 / 23.6 -> 22.0 us; N = 12288 as 96
-    // whole tiles 16.9 -> 17.1 / 22.3 -> 19.7 us.
-    if (tiles < sms && grid == sms) {
-        const long long s_per_tile = sms / tiles;
-        const long long aligned = tiles * (s_per_tile < num_kb ? s_per_tile : num_kb);
-        // S = 1 (whole tiles on 60-90 % of the SMs) trades a longer k loop for no reduction at all: that pays from
-        // 33 rows on (N = 12288: 20.0 us either way at 64 rows, 17.6 us whole against 16.2 us split at 32).
-        const bool whole_tiles = aligned == tiles;
-        if (aligned * 100 >= (long long)sms * 60 && total / aligned >= 4 && (!whole_tiles || a.MB > 32)) grid = aligned;
-    }
-    static const int force_grid = [] { const char *e = getenv("XN_SKINNY_GRID"); return e ? atoi(e) : 0; }();
-    if (force_grid > 0 && force_grid <= sms && force_grid <= total) grid = force_grid;
-    XN_REQUIRE(total < (1ll << 30), "skinny matmul: problem too large for the kernel's 32-bit unit index");
-    a.uq = (int)(total / grid);
-    a.ur = (int)(total % grid);
-    if (int rcw = wait_ctx(&a.wait)) return rcw;
-    a.w_static = (KIND == 0 || rhs_is_static()) ? 1 : 0;  // the fp8 entry points take a static weight by contract
-    SkinnyScratch sc;
-    int rc = skinny_scratch(st, (size_t)2 * grid * a.MB * BM * sizeof(float), (size_t)tiles * 4, &sc);
-    if (rc) return rc;
-    a.partials = sc.partials;
-    a.counters = sc.counters;
-    CUtensorMap mw, mx0, mx1;
-    rc = make_map(&mw, w, ELEM, n, k, ldw, BM);
-    if (rc) return rc;
-    rc = make_map(&mx0, x0, ELEM, m, k, ldx, a.MB);
-    if (rc) return rc;
-    rc = make_map(&mx1, x1 ? x1 : x0, ELEM, m, k, ldx, a.MB);
-    if (rc) return rc;
-    const size_t smem = (size_t)a.nstage * stage + 1024;
-    auto kern = gemm_tcgen05_skinny_kernel<KIND>;
-    XN_ENSURE_SMEM(kern, smem);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(NTHREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    XN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, mw, mx0, mx1, a));
-    return XN_OK;
-}
-
 // y f32 [m, ldy] = x_scale[i] * sum over 32-blocks of scale[j, blk] * (int32 block sum of xq[i] . w8[j]); w8 is the
 // row-major int8 image [n_pad, k] of a q4 / q8 weight, w_scale its [n_pad, k / 32] block scales.
 int launch_gemm_q8_block(float *y, size_t ldy, const int8_t *xq, const float *x_scale, const int8_t *w8, const float *w_scale,
@@ -2006,16 +1377,10 @@ int launch_attention_prefill(xn_dtype dt, void *out, size_t ldo, const void *q, 
     return XN_OK;
 }
 
-int launch_linear_fp8_skinny(void *y, const uint8_t *x_hi, const uint8_t *x_lo, const float *x_scale, const uint8_t *wq,
-                             const float *w_scale, size_t m, size_t n, size_t k, cudaStream_t st) {
-    return launch_skinny<0>(y, n, x_hi, x_lo, k, x_scale, wq, k, w_scale, m, n, k, st);
-}
-
 // y bf16 [m,n] = x_scale[m] * w_scale[n] * (x_hi (+ x_lo)) * wq^T, all operands row-major e4m3.
 int launch_linear_fp8_gemm(void *y, const uint8_t *x_hi, const uint8_t *x_lo, const float *x_scale, const uint8_t *wq,
                            const float *w_scale, size_t m, size_t n, size_t k, cudaStream_t st) {
-    static const size_t skinny_max = [] { const char *e = getenv("XN_FP8_SKINNY_MAX_M"); return e ? (size_t)atoi(e) : (size_t)64; }();
-    if (m <= skinny_max) return launch_linear_fp8_skinny(y, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st);
+    if (gemm_skinny_wanted(m, n, k)) return launch_skinny_fp8(y, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, n, st);
     GemmArgs a{};
     a.y[0] = y; a.ndst = 1; a.col_offset = 0; a.batch = 1; a.y_batch_stride = 0;
     a.x_scale = x_scale; a.w_scale = w_scale; a.M = (int)m; a.N = (int)n; a.K = (int)k; a.ldy = (int)n;
@@ -2050,14 +1415,6 @@ int launch_linear_fp8_gemm_multicast(void *y_mc, size_t ldy, size_t col_offset, 
 int launch_gemm_tn_16bit(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k,
                          size_t lda, size_t ldb, size_t ldd, size_t batch, size_t lhs_bs, size_t rhs_bs, cudaStream_t st,
                          int causal, int causal_off) {
-    // Up to 64 rows, one batch: the skinny form (weights on the tensor-memory lanes, work split at k-stage
-    // granularity over all SMs) -- a tiled launch would have too few tiles and too many MMAs per CTA.
-    static const size_t skinny_max = [] { const char *e = getenv("XN_MM_SKINNY16_MAX_M"); return e ? (size_t)atoi(e) : (size_t)64; }();
-    // (measured on the transformer shapes: always better up to 32 rows; from 33 to 64 only when the tiled kernel
-    // would have fewer 64-column tiles than there are SMs)
-    if (!causal && batch == 1 && m <= skinny_max && (m <= 32 || (m <= 64 && (n + 63) / 64 < (size_t)sm_count())))
-        return dt == XN_BF16 ? launch_skinny<1>(dst, ldd, lhs, nullptr, lda, nullptr, rhs, ldb, nullptr, m, n, k, st)
-                             : launch_skinny<2>(dst, ldd, lhs, nullptr, lda, nullptr, rhs, ldb, nullptr, m, n, k, st);
     GemmArgs a{};
     a.y[0] = dst; a.ndst = 1; a.col_offset = 0; a.batch = (int)batch; a.y_batch_stride = (long long)(m * n);
     a.M = (int)m; a.N = (int)n; a.K = (int)k; a.ldy = (int)ldd;

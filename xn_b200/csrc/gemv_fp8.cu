@@ -98,7 +98,7 @@ linear_fp8_gemv_kernel(__nv_bfloat16 *__restrict__ y, const uint8_t *__restrict_
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int row_m = 8 * mt + 2 * t + e;
-                    xs_reg[mt][e] = row_m < m ? __ldg(x_scale + row_m) : 0.0f;
+                    xs_reg[mt][e] = row_m < m ? ld_act_f32(x_scale + row_m) : 0.0f;
                 }
             ws_reg[0] = valid ? __ldg(w_scale + r0) : 0.0f;
             ws_reg[1] = valid ? __ldg(w_scale + r1) : 0.0f;
@@ -205,18 +205,12 @@ int launch(__nv_bfloat16 *y, const uint8_t *x_hi, const uint8_t *x_lo, const flo
 
 }  // namespace
 
-// y [m,n] bf16 from row-major e4m3 pieces; m <= 32.
+// y [m,n] bf16 from row-major e4m3 pieces; m <= 8.
 int launch_linear_fp8_gemv(void *y, const uint8_t *x_hi, const uint8_t *x_lo, const float *x_scale,
                            const uint8_t *wq, const float *w_scale, int m, size_t n, int k, cudaStream_t st) {
     __nv_bfloat16 *yy = (__nv_bfloat16 *)y;
-    if (m <= 8)
-        return x_lo ? launch<1, true>(yy, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st)
-                    : launch<1, false>(yy, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st);
-    if (m <= 16)
-        return x_lo ? launch<2, true>(yy, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st)
-                    : launch<2, false>(yy, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st);
-    return x_lo ? launch<4, true>(yy, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st)
-                : launch<4, false>(yy, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st);
+    return x_lo ? launch<1, true>(yy, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st)
+                : launch<1, false>(yy, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st);
 }
 
 }  // namespace xn

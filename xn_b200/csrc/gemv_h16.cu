@@ -53,7 +53,7 @@ __host__ __device__ inline int h_pitch(int kc) { return (kc + 63) / 64 * 128 + 6
 template <typename T, int MT>
 __global__ void __launch_bounds__(H_WARPS * 32, 1)
 gemv_h16_kernel(T *__restrict__ y, const T *__restrict__ x, const T *__restrict__ w, int m, size_t n, int k, size_t ldy,
-                size_t ldx, size_t ldw, int kchunk, int tiles, int tpc, int ksplit, int w_static) {
+                size_t ldx, size_t ldw, int kchunk, int tiles, int tpc, int ksplit, int w_static, const T *__restrict__ bias) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int RS = h_pitch(kchunk);
     unsigned char *sX = smem;  // MT*8 rows of 16-bit elements
@@ -150,13 +150,17 @@ gemv_h16_kernel(T *__restrict__ y, const T *__restrict__ x, const T *__restrict_
             for (int i = 0; i < 4; ++i) {
                 const size_t row_n = (size_t)tile * 16 + g + 8 * (i >> 1);
                 const int row_m = 8 * mt + 2 * t + (i & 1);
-                if (row_n < n && row_m < m) y[(size_t)row_m * ldy + row_n] = from_f32<T>(acc[mt][i]);
+                if (row_n < n && row_m < m) {
+                    T v = from_f32<T>(acc[mt][i]);
+                    if (bias) v = from_f32<T>(to_f32(v) + to_f32(bias[row_n]));  // nn::Linear: added to the rounded product
+                    y[(size_t)row_m * ldy + row_n] = v;
+                }
             }
     }
 }
 
 template <typename T, int MT>
-int launch(T *y, const T *x, const T *w, int m, size_t n, int k, size_t ldy, size_t ldx, size_t ldw, cudaStream_t st) {
+int launch(T *y, const T *x, const T *w, int m, size_t n, int k, size_t ldy, size_t ldx, size_t ldw, const T *bias, cudaStream_t st) {
     const int tiles = (int)((n + 15) / 16);
     const int sms = sm_count();
     int tpc = (tiles + sms - 1) / sms;
@@ -183,17 +187,17 @@ int launch(T *y, const T *x, const T *w, int m, size_t n, int k, size_t ldy, siz
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    XN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, y, x, w, m, n, k, ldy, ldx, ldw, kchunk, tiles, tpc, ksplit, rhs_is_static() ? 1 : 0));
+    XN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, y, x, w, m, n, k, ldy, ldx, ldw, kchunk, tiles, tpc, ksplit, rhs_is_static() ? 1 : 0, bias));
     return XN_OK;
 }
 
 template <typename T>
 int launch_t(void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k, size_t dst_rs, size_t lhs_rs,
-             size_t rhs_cs, cudaStream_t st) {
+             size_t rhs_cs, const void *bias, cudaStream_t st) {
     T *y = (T *)dst;
-    const T *x = (const T *)lhs, *w = (const T *)rhs;
-    if (m <= 8) return launch<T, 1>(y, x, w, (int)m, n, (int)k, dst_rs, lhs_rs, rhs_cs, st);
-    return launch<T, 2>(y, x, w, (int)m, n, (int)k, dst_rs, lhs_rs, rhs_cs, st);
+    const T *x = (const T *)lhs, *w = (const T *)rhs, *b = (const T *)bias;
+    if (m <= 8) return launch<T, 1>(y, x, w, (int)m, n, (int)k, dst_rs, lhs_rs, rhs_cs, b, st);
+    return launch<T, 2>(y, x, w, (int)m, n, (int)k, dst_rs, lhs_rs, rhs_cs, b, st);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -364,9 +368,9 @@ bool gemv_h16_single_chunk(size_t m, size_t k) {
 // Caller guarantees: f16 or bf16, m <= 16, one batch, k a multiple of 8, lhs/rhs k-contiguous with pitches that
 // are multiples of 8 elements, 16-byte aligned bases, dst rows contiguous.
 int launch_gemv_h16(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k, size_t dst_rs,
-                    size_t lhs_rs, size_t rhs_cs, cudaStream_t st) {
-    if (dt == XN_F16) return launch_t<__half>(dst, lhs, rhs, m, n, k, dst_rs, lhs_rs, rhs_cs, st);
-    return launch_t<__nv_bfloat16>(dst, lhs, rhs, m, n, k, dst_rs, lhs_rs, rhs_cs, st);
+                    size_t lhs_rs, size_t rhs_cs, const void *bias, cudaStream_t st) {
+    if (dt == XN_F16) return launch_t<__half>(dst, lhs, rhs, m, n, k, dst_rs, lhs_rs, rhs_cs, bias, st);
+    return launch_t<__nv_bfloat16>(dst, lhs, rhs, m, n, k, dst_rs, lhs_rs, rhs_cs, bias, st);
 }
 
 // What the batched kernel takes beyond the alignment rules below: both operands' staged rows within half an SM's

@@ -69,8 +69,7 @@ gemv_kn16_kernel(T *__restrict__ y, const T *__restrict__ x, const T *__restrict
     // cw (1 or 2) strips of 64 columns per CTA, kw warps along k per strip
     const int kw = KN_WARPS / cw, wk = warp & (kw - 1), wc = warp / kw;
     const int b = (int)(strip_id / strips), j0 = ((int)(strip_id - (long long)b * strips) * cw + wc) * KN_COLS;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    dependent_begin();
 
     const T *X = x + (size_t)b * xb;
     const int col = j0 + 8 * g;                       // this lane's 8 output columns
@@ -113,7 +112,7 @@ gemv_kn16_kernel(T *__restrict__ y, const T *__restrict__ x, const T *__restrict
             for (int idx = tid; idx < m * cols8; idx += KN_WARPS * 32) {
                 const int row = (int)((unsigned)idx / (unsigned)cols8), c = idx - row * cols8;
                 uint4 e = make_uint4(0, 0, 0, 0);
-                if (c * 8 < cn) e = *reinterpret_cast<const uint4 *>(X + (size_t)row * ldx + c0 + c * 8);
+                if (c * 8 < cn) e = ld_act128(X + (size_t)row * ldx + c0 + c * 8);
                 *reinterpret_cast<uint4 *>(sX + (size_t)row * RS + c * 16) = e;
             }
         } else {  // any row pitch: a context has whatever length it has; eight loads in flight per thread
@@ -125,7 +124,7 @@ gemv_kn16_kernel(T *__restrict__ y, const T *__restrict__ x, const T *__restrict
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
                         const int c = cb + q * KN_WARPS * 32;
-                        e[q] = c < cn ? __ldg(Xe + (size_t)row * ldx + c) : (unsigned short)0;
+                        e[q] = c < cn ? ld_act_u16(Xe + (size_t)row * ldx + c) : (unsigned short)0;
                     }
 #pragma unroll
                     for (int q = 0; q < 8; ++q) {
@@ -271,14 +270,13 @@ int launch(T *y, const T *x, const T *w, int m, size_t n, size_t k, size_t batch
 
 // dst rows at a pitch of `ldd` elements, the columns [k, ldd) left as they are
 __global__ void __launch_bounds__(256)
-repitch_rows_kernel(unsigned short *__restrict__ dst, const unsigned short *__restrict__ src, size_t rows, size_t m, int k, int ldd,
+repitch_rows_kernel(unsigned short *dst, const unsigned short *src, size_t rows, size_t m, int k, int ldd,
                     size_t lds, size_t src_bs) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    dependent_begin();
     for (size_t r = (size_t)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (size_t)gridDim.x * 8) {
         const unsigned short *s = src + r / m * src_bs + r % m * lds;
         unsigned short *d = dst + r * ldd;
-        for (int c = threadIdx.x & 31; c < k; c += 32) d[c] = s[c];
+        for (int c = threadIdx.x & 31; c < k; c += 32) d[c] = ld_act_u16(s + c);
     }
 }
 

@@ -211,7 +211,7 @@ linear_q4_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const flo
 #pragma unroll
         for (int e = 0; e < 2; ++e) {
             const int row_m = 8 * mt + 2 * t + e;
-            xs_reg[mt][e] = row_m < m ? __ldg(x_scale + row_m) : 0.0f;
+            xs_reg[mt][e] = row_m < m ? ld_act_f32(x_scale + row_m) : 0.0f;
         }
     // The rest of the first ring-full.  With few activation rows it goes out at once.  From 6 rows on the
     // activation copies (24+ KB per SM, wanted before any MMA can start) would share the SM's copy
@@ -389,8 +389,8 @@ linear_q_tile_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const
             const unsigned *src = reinterpret_cast<const unsigned *>(xrow[mt] + (size_t)i * 128);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                b[mt][2 * j] = __ldg(src + 8 * j);
-                b[mt][2 * j + 1] = __ldg(src + 8 * j + 4);
+                b[mt][2 * j] = __float_as_uint(ld_act_f32(reinterpret_cast<const float *>(src + 8 * j)));
+                b[mt][2 * j + 1] = __float_as_uint(ld_act_f32(reinterpret_cast<const float *>(src + 8 * j + 4)));
             }
         }
     };
@@ -455,7 +455,7 @@ linear_q_tile_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const
                 const size_t row_n = (size_t)tile * 16 + g + 8 * (e >> 1);
                 const int row_m = 8 * mt + 2 * t + (e & 1);
                 if (row_n < n && row_m < m)
-                    y[(size_t)row_m * n + row_n] = __ldg(x_scale + row_m) * (acc[mt][e] * (BITS == 4 ? 0.0625f : 1.0f));
+                    y[(size_t)row_m * n + row_n] = ld_act_f32(x_scale + row_m) * (acc[mt][e] * (BITS == 4 ? 0.0625f : 1.0f));
             }
     }
 }

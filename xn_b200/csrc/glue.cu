@@ -148,155 +148,216 @@ template <> __device__ __forceinline__ unsigned max2<__half>(unsigned a, unsigne
     const __half2 r = __hmax2(*reinterpret_cast<const __half2 *>(&a), *reinterpret_cast<const __half2 *>(&b));
     return *reinterpret_cast<const unsigned *>(&r);
 }
-// the e4m3 pieces of eight values already divided by the row scale
-__device__ __forceinline__ void store_pieces8(uint8_t *hi, uint8_t *lo, size_t off, const float (&yv)[8]) {
-    uint8_t h[8], l[8];
+// The e4m3 pieces of eight 16-bit values times `inv` (a power of two): hi = e4m3(v), lo = e4m3(v - hi), in pairs.
+template <typename T>
+__device__ __forceinline__ void store_pieces8(uint8_t *hi, uint8_t *lo, size_t off, const uint4 &v, float inv) {
+    const unsigned w[4] = {v.x, v.y, v.z, v.w};
+    unsigned short h[4], l[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        h[j] = (uint8_t)__nv_cvt_float_to_fp8(yv[j], __NV_SATFINITE, __NV_E4M3);
-        l[j] = (uint8_t)__nv_cvt_float_to_fp8(yv[j] - e4m3_f32(h[j]), __NV_SATFINITE, __NV_E4M3);
+    for (int j = 0; j < 4; ++j) {
+        float2 f = unpack2<T>(w[j]);
+        f.x *= inv;
+        f.y *= inv;
+        h[j] = __nv_cvt_float2_to_fp8x2(f, __NV_SATFINITE, __NV_E4M3);
+        if (lo) {
+            const __half2_raw b = __nv_cvt_fp8x2_to_halfraw2(h[j], __NV_E4M3);
+            const float2 g = __half22float2(__half2(b));
+            l[j] = __nv_cvt_float2_to_fp8x2(make_float2(f.x - g.x, f.y - g.y), __NV_SATFINITE, __NV_E4M3);
+        }
     }
-    *reinterpret_cast<uint2 *>(hi + off) = *reinterpret_cast<const uint2 *>(h);
-    if (lo) *reinterpret_cast<uint2 *>(lo + off) = *reinterpret_cast<const uint2 *>(l);
+    *reinterpret_cast<uint2 *>(hi + off) = make_uint2(h[0] | (unsigned)h[1] << 16, h[2] | (unsigned)h[3] << 16);
+    if (lo) *reinterpret_cast<uint2 *>(lo + off) = make_uint2(l[0] | (unsigned)l[1] << 16, l[2] | (unsigned)l[3] << 16);
 }
 
+// One barrier: every warp leaves its value in `red` and reduces all of them again (`red` must not be in use by another
+// reduction of the same kernel).
+__device__ __forceinline__ float block_sum_once(float v, float *red) {
+    v = warp_sum(v);
+    const int lane = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+    if (lane == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    return warp_sum(lane < nw ? red[lane] : 0.0f);
+}
+__device__ __forceinline__ float block_max_once(float v, float *red) {
+    v = warp_max(v);
+    const int lane = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+    if (lane == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    return warp_max(lane < nw ? red[lane] : -INFINITY);
+}
+
+// The vector kernels run with few threads and VPT = 4 vectors each when there are rows enough to fill the machine (many
+// loads per thread in flight, cheap barriers), and with a vector per thread when a decode step brings a handful of rows
+// and the kernel is one chain of latencies.  4096 rows, bf16 with both pieces: rms_norm + residual of 4096 columns 52 ->
+// 30 us (21 us without), gating to 11264 channels 126 -> 81 us; conversions in pairs and one division per row instead of one
+// per element are the other half of it.
 template <typename T, int VPT, bool SPLIT>
 __global__ void __launch_bounds__(NTV)
-rms_norm_vec_kernel(T *__restrict__ dst, uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, float *__restrict__ scale,
-                    const T *__restrict__ src, const T *__restrict__ alpha, int cols, float eps, const T *__restrict__ res,
-                    T *sum_out) {
-    __shared__ float red[32];
+rms_norm_vec_kernel(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T *src, const T *__restrict__ alpha, int cols, float eps,
+                    const T *res, T *sum_out) {
+    __shared__ float red[2][32];
+    dependent_begin();
     const size_t row = blockIdx.x, base = row * (size_t)cols;
     const int nvec = cols / 8;
-    uint4 v[VPT];
+    uint4 v[VPT], r[VPT];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int idx = i * (int)blockDim.x + (int)threadIdx.x;
+        v[i] = r[i] = make_uint4(0, 0, 0, 0);
+        if (idx < nvec) {
+            v[i] = ld_act128(reinterpret_cast<const uint4 *>(src + base) + idx);
+            if (res) r[i] = ld_act128(reinterpret_cast<const uint4 *>(res + base) + idx);
+        }
+    }
     float s2 = 0.0f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-        const int idx = i * NTV + threadIdx.x;
-        if (idx >= nvec) { v[i] = make_uint4(0, 0, 0, 0); continue; }
-        v[i] = __ldg(reinterpret_cast<const uint4 *>(src + base) + idx);
-        float f[8];
-        unpack8<T>(v[i], f);
-        if (res) {
-            float r[8];
-            unpack8<T>(__ldg(reinterpret_cast<const uint4 *>(res + base) + idx), r);
-            T sum[8];
+        const int idx = i * (int)blockDim.x + (int)threadIdx.x;
+        unsigned *w = reinterpret_cast<unsigned *>(&v[i]);
+        const unsigned *q = reinterpret_cast<const unsigned *>(&r[i]);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) { sum[j] = from_f32<T>(f[j] + r[j]); f[j] = to_f32(sum[j]); }
-            v[i] = pack8<T>(sum);
-            reinterpret_cast<uint4 *>(sum_out + base)[idx] = v[i];
+        for (int j = 0; j < 4; ++j) {
+            float2 f = unpack2<T>(w[j]);
+            if (res) {
+                const float2 g = unpack2<T>(q[j]);
+                w[j] = pack2<T>(f.x + g.x, f.y + g.y);
+                f = unpack2<T>(w[j]);
+            }
+            s2 += f.x * f.x;
+            s2 += f.y * f.y;
         }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) s2 += f[j] * f[j];
+        if (res && idx < nvec) reinterpret_cast<uint4 *>(sum_out + base)[idx] = v[i];
     }
-    s2 = block_sum(s2, red);
-    const float denom = sqrtf(s2 / (float)cols + eps);
+    s2 = block_sum_once(s2, red[0]);
+    const float denom = sqrtf(s2 / (float)cols + eps), rden = __frcp_rn(denom);
+    // x / denom for every element from the row's one reciprocal: with rden = RN(1 / denom), q = x * rden and the residual
+    // x - q * denom (exact in an fma), q + residual * rden is the correctly rounded quotient (Markstein's theorem on
+    // division by a correctly rounded reciprocal; outside the subnormal range).
+    auto quotient = [&](float x) {
+        const float q = x * rden;
+        return fmaf(fmaf(-q, denom, x), rden, q);
+    };
     float amax = 0.0f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-        const int idx = i * NTV + threadIdx.x;
+        const int idx = i * (int)blockDim.x + (int)threadIdx.x;
         if (idx >= nvec) continue;
-        float f[8], al[8];
-        unpack8<T>(v[i], f);
-        unpack8<T>(__ldg(reinterpret_cast<const uint4 *>(alpha) + idx), al);
-        T y[8];
+        const uint4 al = __ldg(reinterpret_cast<const uint4 *>(alpha) + idx);
+        unsigned *w = reinterpret_cast<unsigned *>(&v[i]);
+        const unsigned *q = reinterpret_cast<const unsigned *>(&al);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            y[j] = from_f32<T>(f[j] / denom * al[j]);
-            if (SPLIT) amax = fmaxf(amax, fabsf(to_f32(y[j])));
+        for (int j = 0; j < 4; ++j) {
+            const float2 f = unpack2<T>(w[j]), g = unpack2<T>(q[j]);
+            w[j] = pack2<T>(quotient(f.x) * g.x, quotient(f.y) * g.y);
+            if (SPLIT) {
+                const float2 y = unpack2<T>(w[j]);
+                amax = fmaxf(amax, fmaxf(fabsf(y.x), fabsf(y.y)));
+            }
         }
-        v[i] = pack8<T>(y);
         if (dst) reinterpret_cast<uint4 *>(dst + base)[idx] = v[i];
     }
     if (SPLIT) {
-        amax = block_max2(amax, red);
+        amax = block_max_once(amax, red[1]);
         const float sc = pow2_scale(amax), inv = 1.0f / sc;
         if (threadIdx.x == 0) scale[row] = sc;
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
-            const int idx = i * NTV + threadIdx.x;
-            if (idx >= nvec) continue;
-            float f[8];
-            unpack8<T>(v[i], f);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] *= inv;
-            store_pieces8(hi, lo, base + (size_t)idx * 8, f);
+            const int idx = i * (int)blockDim.x + (int)threadIdx.x;
+            if (idx < nvec) store_pieces8<T>(hi, lo, base + (size_t)idx * 8, v[i], inv);
         }
     }
 }
 
 template <typename T, int VPT, bool SPLIT>
 __global__ void __launch_bounds__(NTV)
-silu_mul_vec_kernel(T *__restrict__ dst, uint8_t *__restrict__ hi, uint8_t *__restrict__ lo, float *__restrict__ scale,
-                    const T *__restrict__ src, int hidden) {
+silu_mul_vec_kernel(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T *src, int hidden) {
     __shared__ float red[32];
+    dependent_begin();
     const size_t row = blockIdx.x, obase = row * (size_t)hidden;
     const uint4 *a = reinterpret_cast<const uint4 *>(src + row * 2 * (size_t)hidden);
     const uint4 *b = reinterpret_cast<const uint4 *>(src + row * 2 * (size_t)hidden + hidden);
     const int nvec = hidden / 8;
-    uint4 v[VPT];
+    uint4 v[VPT], g[VPT];
+#pragma unroll
+    for (int i = 0; i < VPT; ++i) {
+        const int idx = i * (int)blockDim.x + (int)threadIdx.x;
+        v[i] = g[i] = make_uint4(0, 0, 0, 0);
+        if (idx < nvec) {
+            v[i] = ld_act128(a + idx);
+            g[i] = ld_act128(b + idx);
+        }
+    }
+    auto silu = [](float x) { return x / (1.0f + expf(-x)); };
     float amax = 0.0f;
 #pragma unroll
     for (int i = 0; i < VPT; ++i) {
-        const int idx = i * NTV + threadIdx.x;
-        if (idx >= nvec) { v[i] = make_uint4(0, 0, 0, 0); continue; }
-        float av[8], bv[8];
-        unpack8<T>(__ldg(a + idx), av);
-        unpack8<T>(__ldg(b + idx), bv);
-        T y[8];
+        const int idx = i * (int)blockDim.x + (int)threadIdx.x;
+        if (idx >= nvec) continue;
+        unsigned *w = reinterpret_cast<unsigned *>(&v[i]);
+        const unsigned *q = reinterpret_cast<const unsigned *>(&g[i]);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float sl = to_f32(from_f32<T>(av[j] / (1.0f + expf(-av[j]))));
-            y[j] = from_f32<T>(sl * bv[j]);
-            if (SPLIT) amax = fmaxf(amax, fabsf(to_f32(y[j])));
+        for (int j = 0; j < 4; ++j) {
+            const float2 f = unpack2<T>(w[j]), u = unpack2<T>(q[j]);
+            const float2 sl = unpack2<T>(pack2<T>(silu(f.x), silu(f.y)));
+            w[j] = pack2<T>(sl.x * u.x, sl.y * u.y);
+            if (SPLIT) {
+                const float2 y = unpack2<T>(w[j]);
+                amax = fmaxf(amax, fmaxf(fabsf(y.x), fabsf(y.y)));
+            }
         }
-        v[i] = pack8<T>(y);
         if (dst) reinterpret_cast<uint4 *>(dst + obase)[idx] = v[i];
     }
     if (SPLIT) {
-        amax = block_max2(amax, red);
+        amax = block_max_once(amax, red);
         const float sc = pow2_scale(amax), inv = 1.0f / sc;
         if (threadIdx.x == 0) scale[row] = sc;
 #pragma unroll
         for (int i = 0; i < VPT; ++i) {
-            const int idx = i * NTV + threadIdx.x;
-            if (idx >= nvec) continue;
-            float f[8];
-            unpack8<T>(v[i], f);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) f[j] *= inv;
-            store_pieces8(hi, lo, obase + (size_t)idx * 8, f);
+            const int idx = i * (int)blockDim.x + (int)threadIdx.x;
+            if (idx < nvec) store_pieces8<T>(hi, lo, obase + (size_t)idx * 8, v[i], inv);
         }
     }
 }
 
 // Picks the vector kernels for 16-bit rows that fit (8-element vectors, 16-byte aligned rows); returns false when the
 // scalar kernel has to run.
-template <typename T, bool SPLIT>
-bool launch_rms_norm_vec(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T *src, const T *alpha, size_t rows, size_t cols,
-                         float eps, const T *res, T *sum_out, cudaStream_t st) {
-    if (sizeof(T) != 2 || cols % 8 != 0 || cols > (size_t)NTV * 8 * 4 || !aligned(src, 16) || !aligned(alpha, 16) ||
-        (dst && !aligned(dst, 16)) || (res && (!aligned(res, 16) || !aligned(sum_out, 16))) || (hi && !aligned(hi, 8)) ||
-        (lo && !aligned(lo, 8)))
-        return false;
-    if (cols <= (size_t)NTV * 8)
-        rms_norm_vec_kernel<T, 1, SPLIT><<<(unsigned)rows, NTV, 0, st>>>(dst, hi, lo, scale, src, alpha, (int)cols, eps, res, sum_out);
-    else
-        rms_norm_vec_kernel<T, 4, SPLIT><<<(unsigned)rows, NTV, 0, st>>>(dst, hi, lo, scale, src, alpha, (int)cols, eps, res, sum_out);
-    return true;
+struct RowShape { int vpt; unsigned threads; };
+inline RowShape row_shape(size_t rows, size_t nvec) {
+    // rows for two rounds of the machine at least: four vectors per thread
+    if (rows >= (size_t)sm_count() * 4 && nvec <= NTV * 4) return {4, (unsigned)((nvec + 127) / 128 * 32)};
+    if (nvec <= NTV) return {1, (unsigned)((nvec + 31) / 32 * 32)};
+    return {nvec <= NTV * 4 ? 4 : 8, NTV};
 }
 template <typename T, bool SPLIT>
-bool launch_silu_mul_vec(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T *src, size_t rows, size_t hidden, cudaStream_t st) {
-    if (sizeof(T) != 2 || hidden % 8 != 0 || hidden > (size_t)NTV * 8 * 8 || !aligned(src, 16) || (dst && !aligned(dst, 16)) ||
-        (hi && !aligned(hi, 8)) || (lo && !aligned(lo, 8)))
-        return false;
-    if (hidden <= (size_t)NTV * 8)
-        silu_mul_vec_kernel<T, 1, SPLIT><<<(unsigned)rows, NTV, 0, st>>>(dst, hi, lo, scale, src, (int)hidden);
-    else if (hidden <= (size_t)NTV * 8 * 3)
-        silu_mul_vec_kernel<T, 3, SPLIT><<<(unsigned)rows, NTV, 0, st>>>(dst, hi, lo, scale, src, (int)hidden);
-    else
-        silu_mul_vec_kernel<T, 8, SPLIT><<<(unsigned)rows, NTV, 0, st>>>(dst, hi, lo, scale, src, (int)hidden);
-    return true;
+bool launch_rms_norm_vec(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T *src, const T *alpha, size_t rows, size_t cols,
+                         float eps, const T *res, T *sum_out, cudaStream_t st, int *rc) {
+    if constexpr (sizeof(T) == 2) {
+        if (cols % 8 != 0 || cols > (size_t)NTV * 8 * 4 || !aligned(src, 16) || !aligned(alpha, 16) || (dst && !aligned(dst, 16)) ||
+            (res && (!aligned(res, 16) || !aligned(sum_out, 16))) || (hi && !aligned(hi, 8)) || (lo && !aligned(lo, 8)))
+            return false;
+        const RowShape sh = row_shape(rows, cols / 8);
+        auto kern = sh.vpt == 1 ? rms_norm_vec_kernel<T, 1, SPLIT> : rms_norm_vec_kernel<T, 4, SPLIT>;
+        *rc = launch_dependent(kern, dim3((unsigned)rows), dim3(sh.threads), 0, st, dst, hi, lo, scale, src, alpha, (int)cols, eps, res,
+                               sum_out);
+        return true;
+    }
+    return false;
+}
+template <typename T, bool SPLIT>
+bool launch_silu_mul_vec(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T *src, size_t rows, size_t hidden, cudaStream_t st,
+                         int *rc) {
+    if constexpr (sizeof(T) == 2) {
+        if (hidden % 8 != 0 || hidden > (size_t)NTV * 8 * 8 || !aligned(src, 16) || (dst && !aligned(dst, 16)) ||
+            (hi && !aligned(hi, 8)) || (lo && !aligned(lo, 8)))
+            return false;
+        const RowShape sh = row_shape(rows, hidden / 8);
+        auto kern = sh.vpt == 1   ? silu_mul_vec_kernel<T, 1, SPLIT>
+                    : sh.vpt == 4 ? silu_mul_vec_kernel<T, 4, SPLIT>
+                                  : silu_mul_vec_kernel<T, 8, SPLIT>;
+        *rc = launch_dependent(kern, dim3((unsigned)rows), dim3(sh.threads), 0, st, dst, hi, lo, scale, src, (int)hidden);
+        return true;
+    }
+    return false;
 }
 
 // The row in registers, one CTA per row, one read and one write: max-subtract, exp rounded to T, f32 sum of the rounded
@@ -306,11 +367,10 @@ bool launch_silu_mul_vec(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T
 // 21.7 us for 256 rows of 1501, now 2.4 us.
 template <typename T, int VPT>
 __global__ void __launch_bounds__(256)
-softmax_row_kernel(T *__restrict__ dst, const T *__restrict__ src, int cols) {
+softmax_row_kernel(T *dst, const T *src, int cols) {
     constexpr int V = 16 / (int)sizeof(T);
     __shared__ float red[32];
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    dependent_begin();
     const size_t row = blockIdx.x;
     const T *x = src + row * cols;
     T *y = dst + row * cols;
@@ -319,14 +379,14 @@ softmax_row_kernel(T *__restrict__ dst, const T *__restrict__ src, int cols) {
     // edge element of this thread: the first V lie before the middle, the next V behind it
     const int e = threadIdx.x < (unsigned)V ? (int)threadIdx.x : tail0 + (int)threadIdx.x - V;
     const bool edge = threadIdx.x < (unsigned)V ? e < head : (threadIdx.x < 2u * V && e < cols);
-    float ev = edge ? to_f32(x[e]) : -INFINITY, v[VPT][V];
+    float ev = edge ? to_f32(ld_act(x + e)) : -INFINITY, v[VPT][V];
     float mx = ev;
     const uint4 *xv = reinterpret_cast<const uint4 *>(x + head);
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
         const int idx = u * (int)blockDim.x + (int)threadIdx.x;
         if (idx < nvec) {
-            const uint4 q = xv[idx];
+            const uint4 q = ld_act128(xv + idx);
             const T *el = reinterpret_cast<const T *>(&q);
 #pragma unroll
             for (int j = 0; j < V; ++j) mx = fmaxf(mx, v[u][j] = to_f32(el[j]));
@@ -418,8 +478,31 @@ __global__ void add_kernel(T *__restrict__ dst, const T *__restrict__ a, const T
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < len) dst[i] = from_f32<T>(to_f32(a[i]) + to_f32(b[i]));
 }
+// 16-byte pieces, two per thread in flight (dst may be a or b); the scalar form above took 62 us for 4096 x 4096 bf16.
+template <typename T>
+__global__ void __launch_bounds__(256) add_vec_kernel(T *dst, const T *a, const T *b, size_t nvec) {
+    constexpr int V = 16 / (int)sizeof(T);
+    dependent_begin();
+    const size_t i0 = (size_t)blockIdx.x * 512 + threadIdx.x;
+    uint4 va[2], vb[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+        if (i0 + 256 * u < nvec) {
+            va[u] = ld_act128(reinterpret_cast<const uint4 *>(a) + i0 + 256 * u);
+            vb[u] = ld_act128(reinterpret_cast<const uint4 *>(b) + i0 + 256 * u);
+        }
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+        if (i0 + 256 * u < nvec) {
+            const T *x = reinterpret_cast<const T *>(&va[u]), *y = reinterpret_cast<const T *>(&vb[u]);
+            uint4 r;
+            T *o = reinterpret_cast<T *>(&r);
+#pragma unroll
+            for (int j = 0; j < V; ++j) o[j] = from_f32<T>(to_f32(x[j]) + to_f32(y[j]));
+            reinterpret_cast<uint4 *>(dst)[i0 + 256 * u] = r;
+        }
+}
 
-// cache [batch, heads, context, hd] <- src [batch, heads, 1, hd] at context index idx[batch].
 template <typename T>
 __global__ void kv_append_kernel(T *__restrict__ cache, const T *__restrict__ src, const int64_t *__restrict__ idx,
                                  size_t heads, size_t context, size_t hd, size_t src_batch_stride, size_t total) {
@@ -439,10 +522,10 @@ constexpr int HD = 128;
 // instantiation because the sliced form's extra bounds cost the one-pass case 6 % when they are run-time values.
 template <bool SLICED>
 __global__ void __launch_bounds__(128)
-decode_attention_kernel(__nv_bfloat16 *__restrict__ out, const __nv_bfloat16 *__restrict__ q,
-                        const __nv_bfloat16 *__restrict__ kc, const __nv_bfloat16 *__restrict__ vc,
-                        const float *__restrict__ mask, size_t heads, size_t context, size_t q_batch_stride,
-                        float scale, size_t rows_per_split, float *__restrict__ partial) {
+decode_attention_kernel(__nv_bfloat16 *__restrict__ out, const __nv_bfloat16 *q, const __nv_bfloat16 *kc, const __nv_bfloat16 *vc,
+                        const float *mask, size_t heads, size_t context, size_t q_batch_stride, float scale, size_t rows_per_split,
+                        float *__restrict__ partial) {
+    dependent_begin();
     // blockIdx.y = slice of the context (rows [row_lo, row_hi)); with one slice the result goes straight to `out`,
     // otherwise the slice's running maximum, sum and unnormalised output go to `partial` for the combine kernel
     const size_t bh = blockIdx.x, b = bh / heads;
@@ -453,7 +536,7 @@ decode_attention_kernel(__nv_bfloat16 *__restrict__ out, const __nv_bfloat16 *__
     const int group = warp * 2 + half;  // 8 half-warps stride over the rows
     float qv[8];
     {
-        const uint4 t = *reinterpret_cast<const uint4 *>(q + b * q_batch_stride + (bh % heads) * HD + l16 * 8);
+        const uint4 t = ld_act128(q + b * q_batch_stride + (bh % heads) * HD + l16 * 8);
         const __nv_bfloat16 *e = reinterpret_cast<const __nv_bfloat16 *>(&t);
 #pragma unroll
         for (int j = 0; j < 8; ++j) qv[j] = __bfloat162float(e[j]) * scale;
@@ -548,8 +631,8 @@ decode_attention_kernel(__nv_bfloat16 *__restrict__ out, const __nv_bfloat16 *__
 // Log-sum-exp merge of the context slices of one (stream, head): out = sum_s w_s o_s / sum_s w_s l_s,
 // w_s = exp(m_s - max_s m_s).  One CTA of 128 threads per (stream, head).
 __global__ void __launch_bounds__(HD)
-decode_attention_combine_kernel(__nv_bfloat16 *__restrict__ out, const float *__restrict__ partial, int splits) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+decode_attention_combine_kernel(__nv_bfloat16 *out, const float *partial, int splits) {
+    dependent_begin();
     const size_t bh = blockIdx.x;
     const float *p = partial + bh * splits * (HD + 2);
     float mx = -INFINITY;
@@ -569,9 +652,9 @@ constexpr int AHD = 128;  // head dimension of the attention kernels
 // the activation of the output projection, whose fp8 pieces need the row's maximum over all heads.  One CTA of
 // 1024 threads per stream; a thread owns 4 consecutive dimensions of up to two heads (heads <= 64).
 __global__ void __launch_bounds__(1024)
-decode_attention_combine_split_kernel(__nv_bfloat16 *__restrict__ out, uint8_t *__restrict__ hi, uint8_t *__restrict__ lo,
-                                      float *__restrict__ xs, const float *__restrict__ partial, int splits, int heads) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+decode_attention_combine_split_kernel(__nv_bfloat16 *out, uint8_t *hi, uint8_t *lo, float *xs, const float *partial, int splits,
+                                      int heads) {
+    dependent_begin();
     __shared__ float red[32];
     const size_t b = blockIdx.x;
     const int items = heads * (AHD / 4);
@@ -1035,8 +1118,10 @@ extern "C" int xn_mm_rms_norm(xn_dtype dtype, void *dst, const void *src, const 
     XN_REQUIRE(dst && src && alpha, "rms_norm: null pointer");
     XN_REQUIRE(rows <= 0x7fffffffull, "rms_norm: too many rows");
     XN_DISPATCH_DTYPE(dtype, T,
-        if (!launch_rms_norm_vec<T, false>((T *)dst, nullptr, nullptr, nullptr, (const T *)src, (const T *)alpha, rows, cols, eps,
-                                           nullptr, nullptr, (cudaStream_t)stream))
+        if (int rc = XN_OK; launch_rms_norm_vec<T, false>((T *)dst, nullptr, nullptr, nullptr, (const T *)src, (const T *)alpha, rows, cols, eps,
+                                           nullptr, nullptr, (cudaStream_t)stream, &rc))
+            return rc;
+        else
             rms_norm_kernel<T, false><<<(unsigned)rows, NT, 0, (cudaStream_t)stream>>>(
                 (T *)dst, nullptr, nullptr, nullptr, (const T *)src, (const T *)alpha, cols, eps));
     XN_CHECK_CUDA(cudaGetLastError());
@@ -1052,8 +1137,10 @@ extern "C" int xn_mm_rms_norm_split_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_
     XN_REQUIRE(x_hi && x_scale && src && alpha, "rms_norm_split: null pointer");
     XN_REQUIRE(rows <= 0x7fffffffull, "rms_norm_split: too many rows");
     XN_DISPATCH_DTYPE(dtype, T,
-        if (!launch_rms_norm_vec<T, true>((T *)dst_or_null, x_hi, x_lo, x_scale, (const T *)src, (const T *)alpha, rows, cols, eps,
-                                          nullptr, nullptr, (cudaStream_t)stream))
+        if (int rc = XN_OK; launch_rms_norm_vec<T, true>((T *)dst_or_null, x_hi, x_lo, x_scale, (const T *)src, (const T *)alpha, rows, cols, eps,
+                                          nullptr, nullptr, (cudaStream_t)stream, &rc))
+            return rc;
+        else
             rms_norm_kernel<T, true><<<(unsigned)rows, NT, 0, (cudaStream_t)stream>>>(
                 (T *)dst_or_null, x_hi, x_lo, x_scale, (const T *)src, (const T *)alpha, cols, eps));
     XN_CHECK_CUDA(cudaGetLastError());
@@ -1069,8 +1156,10 @@ extern "C" int xn_mm_add_rms_norm_split_e4m3(uint8_t *x_hi, uint8_t *x_lo, float
     XN_REQUIRE(x_hi && x_scale && sum_out && a && b && alpha, "add_rms_norm_split: null pointer");
     XN_REQUIRE(rows <= 0x7fffffffull, "add_rms_norm_split: too many rows");
     XN_DISPATCH_DTYPE(dtype, T,
-        if (!launch_rms_norm_vec<T, true>((T *)nullptr, x_hi, x_lo, x_scale, (const T *)a, (const T *)alpha, rows, cols, eps,
-                                          (const T *)b, (T *)sum_out, (cudaStream_t)stream))
+        if (int rc = XN_OK; launch_rms_norm_vec<T, true>((T *)nullptr, x_hi, x_lo, x_scale, (const T *)a, (const T *)alpha, rows, cols, eps,
+                                          (const T *)b, (T *)sum_out, (cudaStream_t)stream, &rc))
+            return rc;
+        else
             rms_norm_kernel<T, true><<<(unsigned)rows, NT, 0, (cudaStream_t)stream>>>(
                 (T *)nullptr, x_hi, x_lo, x_scale, (const T *)a, (const T *)alpha, cols, eps, (const T *)b, (T *)sum_out));
     XN_CHECK_CUDA(cudaGetLastError());
@@ -1105,7 +1194,9 @@ extern "C" int xn_mm_silu_mul(xn_dtype dtype, void *dst, const void *src, size_t
     XN_REQUIRE(dst && src, "silu_mul: null pointer");
     XN_REQUIRE(rows <= 0x7fffffffull, "silu_mul: too many rows");
     XN_DISPATCH_DTYPE(dtype, T,
-        if (!launch_silu_mul_vec<T, false>((T *)dst, nullptr, nullptr, nullptr, (const T *)src, rows, hidden, (cudaStream_t)stream))
+        if (int rc = XN_OK; launch_silu_mul_vec<T, false>((T *)dst, nullptr, nullptr, nullptr, (const T *)src, rows, hidden, (cudaStream_t)stream, &rc))
+            return rc;
+        else
             silu_mul_kernel<T, false><<<(unsigned)rows, NT, 0, (cudaStream_t)stream>>>(
                 (T *)dst, nullptr, nullptr, nullptr, (const T *)src, hidden));
     XN_CHECK_CUDA(cudaGetLastError());
@@ -1120,7 +1211,9 @@ extern "C" int xn_mm_silu_mul_split_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_
     XN_REQUIRE(x_hi && x_scale && src, "silu_mul_split: null pointer");
     XN_REQUIRE(rows <= 0x7fffffffull, "silu_mul_split: too many rows");
     XN_DISPATCH_DTYPE(dtype, T,
-        if (!launch_silu_mul_vec<T, true>((T *)nullptr, x_hi, x_lo, x_scale, (const T *)src, rows, hidden, (cudaStream_t)stream))
+        if (int rc = XN_OK; launch_silu_mul_vec<T, true>((T *)nullptr, x_hi, x_lo, x_scale, (const T *)src, rows, hidden, (cudaStream_t)stream, &rc))
+            return rc;
+        else
             silu_mul_kernel<T, true><<<(unsigned)rows, NT, 0, (cudaStream_t)stream>>>(
                 (T *)nullptr, x_hi, x_lo, x_scale, (const T *)src, hidden));
     XN_CHECK_CUDA(cudaGetLastError());
@@ -1132,6 +1225,10 @@ extern "C" int xn_mm_add(xn_dtype dtype, void *dst, const void *a, const void *b
     XN_REQUIRE(valid_dtype(dtype), "add: unknown dtype %d", (int)dtype);
     if (len == 0) return XN_OK;
     XN_REQUIRE(dst && a && b, "add: null pointer");
+    const size_t nvec = len * dtype_size(dtype) / 16;
+    if (len * dtype_size(dtype) % 16 == 0 && aligned(dst, 16) && aligned(a, 16) && aligned(b, 16) && (nvec + 511) / 512 <= 0x7fffffffull)
+        XN_DISPATCH_DTYPE(dtype, T, return launch_dependent(add_vec_kernel<T>, dim3((unsigned)((nvec + 511) / 512)), dim3(256), 0,
+                                                            (cudaStream_t)stream, (T *)dst, (const T *)a, (const T *)b, nvec));
     const size_t blocks = (len + 255) / 256;
     XN_REQUIRE(blocks <= 0x7fffffffull, "add: too many elements");
     XN_DISPATCH_DTYPE(dtype, T, add_kernel<T><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
@@ -1145,9 +1242,9 @@ extern "C" int xn_mm_add(xn_dtype dtype, void *dst, const void *a, const void *b
 // reference's binary Add does for f16 / bf16.  dst may alias src.
 // Both caches in one launch: blockIdx.y = 0 appends to the key cache, 1 to the value cache.
 template <typename T>
-__global__ void kv_append2_kernel(T *__restrict__ k_cache, T *__restrict__ v_cache, const T *__restrict__ k_src,
-                                  const T *__restrict__ v_src, const int64_t *__restrict__ idx, size_t heads, size_t context,
-                                  size_t hd, size_t src_batch_stride, size_t total) {
+__global__ void kv_append2_kernel(T *k_cache, T *v_cache, const T *k_src, const T *v_src, const int64_t *idx, size_t heads,
+                                  size_t context, size_t hd, size_t src_batch_stride, size_t total) {
+    dependent_begin();
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
     T *cache = blockIdx.y ? v_cache : k_cache;
@@ -1155,7 +1252,7 @@ __global__ void kv_append2_kernel(T *__restrict__ k_cache, T *__restrict__ v_cac
     const size_t d = i % hd, h = (i / hd) % heads, b = i / (hd * heads);
     const int64_t p = idx[b];
     if (p < 0 || (size_t)p >= context) return;  // out-of-range index: nothing is written
-    cache[((b * heads + h) * context + (size_t)p) * hd + d] = src[b * src_batch_stride + h * hd + d];
+    cache[((b * heads + h) * context + (size_t)p) * hd + d] = ld_act(src + b * src_batch_stride + h * hd + d);
 }
 
 template <typename T>
@@ -1232,16 +1329,23 @@ int decode_attention_impl(void *out_bf16, const void *q_bf16, size_t q_batch_str
     const size_t rows_per_split = ((context + splits - 1) / splits + 31) / 32 * 32;
     splits = (int)((context + rows_per_split - 1) / rows_per_split);
     cudaStream_t st = (cudaStream_t)stream;
+    int rc;
+    // A long sweep starts on an idle machine: beside the tail of a kernel that holds most of an SM's shared memory (the
+    // linear before it) the SM would keep that split for the whole sweep and leave the loads in flight -- 80 KB per SM --
+    // too little L1 to land in.  32 streams x 3000 keys: 257 us per layer started early, 223 us not.  A short one gains
+    // from the overlap instead.
+    const bool early = batch * heads * (size_t)splits <= (size_t)sm_count() * 5 * 2;
     if (splits > 1)
-        decode_attention_kernel<true><<<dim3((unsigned)(batch * heads), (unsigned)splits), 128, 0, st>>>(
-            (__nv_bfloat16 *)out_bf16, (const __nv_bfloat16 *)q_bf16, (const __nv_bfloat16 *)k_cache_bf16,
-            (const __nv_bfloat16 *)v_cache_bf16, mask_or_null, heads, context, q_batch_stride, scale, rows_per_split,
-            (float *)workspace);
+        rc = launch_kernel(early, decode_attention_kernel<true>, dim3((unsigned)(batch * heads), (unsigned)splits), dim3(128), 0, st,
+                              (__nv_bfloat16 *)out_bf16, (const __nv_bfloat16 *)q_bf16, (const __nv_bfloat16 *)k_cache_bf16,
+                              (const __nv_bfloat16 *)v_cache_bf16, mask_or_null, heads, context, q_batch_stride, scale, rows_per_split,
+                              (float *)workspace);
     else
-        decode_attention_kernel<false><<<(unsigned)(batch * heads), 128, 0, st>>>(
-            (__nv_bfloat16 *)out_bf16, (const __nv_bfloat16 *)q_bf16, (const __nv_bfloat16 *)k_cache_bf16,
-            (const __nv_bfloat16 *)v_cache_bf16, mask_or_null, heads, context, q_batch_stride, scale, context, nullptr);
-    XN_CHECK_CUDA(cudaGetLastError());
+        rc = launch_kernel(early, decode_attention_kernel<false>, dim3((unsigned)(batch * heads)), dim3(128), 0, st,
+                              (__nv_bfloat16 *)out_bf16, (const __nv_bfloat16 *)q_bf16, (const __nv_bfloat16 *)k_cache_bf16,
+                              (const __nv_bfloat16 *)v_cache_bf16, mask_or_null, heads, context, q_batch_stride, scale, context,
+                              (float *)nullptr);
+    if (rc) return rc;
     if (splits > 1) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)(batch * heads));
@@ -1304,11 +1408,9 @@ extern "C" int xn_mm_kv_append2(xn_dtype dtype, void *k_cache, void *v_cache, co
     XN_REQUIRE(k_cache && v_cache && k_src && v_src && index, "kv_append2: null pointer");
     const size_t blocks = (total + 255) / 256;
     XN_REQUIRE(blocks <= 0x7fffffffull, "kv_append2: too many elements");
-    XN_DISPATCH_DTYPE(dtype, T, kv_append2_kernel<T><<<dim3((unsigned)blocks, 2), 256, 0, (cudaStream_t)stream>>>(
-                                    (T *)k_cache, (T *)v_cache, (const T *)k_src, (const T *)v_src, index, heads, context, head_dim,
-                                    src_batch_stride, total));
-    XN_CHECK_CUDA(cudaGetLastError());
-    return XN_OK;
+    XN_DISPATCH_DTYPE(dtype, T, return launch_dependent(kv_append2_kernel<T>, dim3((unsigned)blocks, 2), dim3(256), 0, (cudaStream_t)stream,
+                                                        (T *)k_cache, (T *)v_cache, (const T *)k_src, (const T *)v_src, index, heads,
+                                                        context, head_dim, src_batch_stride, total));
 }
 
 extern "C" size_t xn_mm_decode_attention_append_workspace_bytes(size_t batch, size_t heads, size_t context) {

@@ -19,6 +19,10 @@ int launch_linear_fp8_gemm_multicast(void *y_mc, size_t ldy, size_t col_offset, 
                                      const float *x_scale, const uint8_t *wq, const float *w_scale, size_t m, size_t n,
                                      size_t k, cudaStream_t st);
 
+// Below this many weight bytes the mma.sync GEMV beats the tensor-memory kernel at up to 8 rows (us, GEMV / tensor
+// memory, W8A16, one row: 1024 x 1024 2.4 / 3.3, 4096 x 4096 7.3 / 6.8, 12288 x 4096 12.8 / 12.3, 4096 x 11264 13.8 / 11.1).
+static constexpr size_t FP8_GEMV_MAX_WEIGHT = 12u << 20;
+
 static inline size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 }  // namespace xn
 
@@ -35,18 +39,11 @@ extern "C" int xn_mm_linear_fp8_pieces(void *y_bf16, const uint8_t *x_hi, const 
     XN_REQUIRE(aligned(wq, 16) && aligned(x_hi, 16) && (!x_lo || aligned(x_lo, 16)),
                "linear_fp8: weights and activation pieces must be 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    // Up to 8 rows (one MMA column group) stream the weights once through the GEMV kernel; anything larger
-    // goes to the tensor-memory kernels (skinny form up to 64 rows, tiled GEMM beyond), which were measured
-    // faster from 9 rows on for every transformer shape.
-    static const size_t gemv_max_m = [] { const char *e = getenv("XN_FP8_GEMV_MAX_M"); return e ? (size_t)atoi(e) : (size_t)8; }();
-    if (m > gemv_max_m) return launch_linear_fp8_gemm(y_bf16, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st);
-    for (size_t i0 = 0; i0 < m; i0 += 32) {
-        const int mc = (int)((m - i0) < 32 ? (m - i0) : 32);
-        int rc = launch_linear_fp8_gemv((char *)y_bf16 + i0 * n * 2, x_hi + i0 * k, x_lo ? x_lo + i0 * k : nullptr,
-                                        x_scale + i0, wq, w_scale, mc, n, (int)k, st);
-        if (rc) return rc;
-    }
-    return XN_OK;
+    // Up to 8 rows (one MMA column group) of a weight too small to be worth a cluster split stream through the GEMV kernel;
+    // anything larger goes to the tensor-memory kernels.
+    if (m <= 8 && n * k < FP8_GEMV_MAX_WEIGHT)
+        return launch_linear_fp8_gemv(y_bf16, x_hi, x_lo, x_scale, wq, w_scale, (int)m, n, (int)k, st);
+    return launch_linear_fp8_gemm(y_bf16, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st);
 }
 
 extern "C" int xn_mm_linear_fp8_pieces_scatter(void *const *y_dsts, size_t num_dst, size_t ldy, size_t col_offset,
@@ -185,11 +182,6 @@ extern "C" int xn_mm_linear_fp8_noalloc(void *y_bf16, const void *x_bf16, const 
     float *xs = reinterpret_cast<float *>(base + NOALLOC_SCALE_OFFSET);
     rc = xn_mm_split_rows_e4m3(hi, variant == 0 ? lo : nullptr, xs, x_bf16, XN_BF16, m, k, stream);
     if (rc) return rc;
-    // Only kernels that need no scratch of their own: the weight-streaming GEMV up to 32 rows, the tiled
-    // tensor-memory kernel beyond.  (xn_mm_linear_fp8_pieces would pick the skinny kernel from 9 rows on, whose
-    // split-tile hand-over lives in a library-owned buffer that is allocated on first use.)
-    const uint8_t *lo_or_null = variant == 0 ? lo : nullptr;
-    if (m <= 32) return launch_linear_fp8_gemv(y_bf16, hi, lo_or_null, xs, wq, w_scale, (int)m, n, (int)k, (cudaStream_t)stream);
-    void *dst[1] = {y_bf16};
-    return launch_linear_fp8_gemm_scatter(dst, 1, n, 0, hi, lo_or_null, xs, wq, w_scale, m, n, k, (cudaStream_t)stream);
+    // Up to 64 rows no kernel needs scratch of its own: the tensor-memory kernel's split tiles meet in shared memory.
+    return xn_mm_linear_fp8_pieces(y_bf16, hi, variant == 0 ? lo : nullptr, xs, wq, w_scale, m, n, k, stream);
 }
