@@ -65,3 +65,34 @@ def test_softmax_rows_of_any_length(xn, cuda, dtype, rows, cols):
     ref = torch.softmax(x.double(), -1)
     u = U[dtype] if dtype != torch.float32 else cols * 2.0 ** -24
     assert bool(((y.double() - ref).abs() <= 16 * u * ref + 1e-7).all())
+
+
+@pytest.mark.parametrize("how", ["add", "rms_norm", "split"])
+def test_a_weight_written_by_the_call_before(xn, cuda, how):
+    """A Linear may fetch its weight before its dependency wait: not while the row kernel that writes it still runs.
+    Inputs are small integers and the expected product is formed after a synchronisation, so both sides are equal."""
+    g = torch.Generator(device=cuda).manual_seed(5)
+    n, k = 22528, 4096
+    a = torch.randint(-4, 5, (n, k), generator=g, device=cuda).to(torch.bfloat16)
+    x = torch.randint(-4, 5, (1, k), generator=g, device=cuda).to(torch.bfloat16)
+    alpha = torch.ones(k, device=cuda, dtype=torch.bfloat16)
+    for _ in range(8):
+        if how == "split":
+            q, _, s = xn.split_rows_e4m3(a, False)
+            y = xn.linear_fp8(x, q, s)
+            torch.cuda.synchronize()
+            ref = xn.linear_fp8(x, q, s)
+        else:
+            w = xn.ops.add(a, a) if how == "add" else xn.ops.rms_norm(a, alpha, 1e-5)
+            y = xn.Linear(w)(x)
+            torch.cuda.synchronize()
+            ref = xn.Linear(w)(x)
+        torch.cuda.synchronize()
+        assert torch.equal(y, ref)
+        a = a.roll(1, 0)
+        if how == "split":
+            q.zero_()
+        else:
+            w.zero_()
+        torch.cuda.synchronize()
+        del y, ref

@@ -135,11 +135,12 @@ __device__ __forceinline__ uint4 ldg_stream(const void *p) {
     return v;
 }
 
-// Kernels launched with launch_dependent() start with this: the next kernel in the stream may begin its own set-up (and
-// fetch what is static, a linear's weights above all) while this one runs, and nothing is touched before the previous
-// one has finished.
-__device__ __forceinline__ void dependent_begin() {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+// Kernels launched with launch_dependent() start with this: nothing is touched before the previous kernel in the stream
+// has finished.  EARLY lets the next kernel begin its own set-up, and fetch what is static (a linear's weights above all),
+// while this one runs.  That is for outputs nobody uses as a weight (quantized pieces, caches, attention rows): a tensor
+// a caller may hand to a Linear as its weight right away (a sum, a normalised or softmaxed matrix) is written without it.
+template <bool EARLY = true> __device__ __forceinline__ void dependent_begin() {
+    if (EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 // Loads of what the previous kernel in the stream wrote, for kernels that may be resident while it still runs: through
@@ -201,6 +202,8 @@ int launch_gemv_dense(xn_dtype dt, void *dst, const void *lhs, const void *rhs, 
                       size_t lhs_b, size_t lhs_b_stride, size_t rhs_b_stride, size_t dst_rs, size_t lhs_rs, size_t rhs_cs,
                       cudaStream_t st);
 bool gemm_skinny_wanted(size_t m, size_t n, size_t k);
+int split_rows_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_scale, const void *x, xn_dtype dtype, size_t m, size_t k, bool pieces_only,
+                    void *stream);
 int launch_skinny_fp8(void *y, const uint8_t *x_hi, const uint8_t *x_lo, const float *x_scale, const uint8_t *wq,
                       const float *w_scale, size_t m, size_t n, size_t k, size_t ldy, cudaStream_t st);
 int launch_skinny_16bit(xn_dtype dt, void *dst, const void *lhs, const void *rhs, const void *bias, size_t m, size_t n, size_t k,

@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(NTV)
 rms_norm_vec_kernel(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T *src, const T *__restrict__ alpha, int cols, float eps,
                     const T *res, T *sum_out) {
     __shared__ float red[2][32];
-    dependent_begin();
+    dependent_begin<SPLIT>();
     const size_t row = blockIdx.x, base = row * (size_t)cols;
     const int nvec = cols / 8;
     uint4 v[VPT], r[VPT];
@@ -272,7 +272,7 @@ template <typename T, int VPT, bool SPLIT>
 __global__ void __launch_bounds__(NTV)
 silu_mul_vec_kernel(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T *src, int hidden) {
     __shared__ float red[32];
-    dependent_begin();
+    dependent_begin<SPLIT>();
     const size_t row = blockIdx.x, obase = row * (size_t)hidden;
     const uint4 *a = reinterpret_cast<const uint4 *>(src + row * 2 * (size_t)hidden);
     const uint4 *b = reinterpret_cast<const uint4 *>(src + row * 2 * (size_t)hidden + hidden);
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(256)
 softmax_row_kernel(T *dst, const T *src, int cols) {
     constexpr int V = 16 / (int)sizeof(T);
     __shared__ float red[32];
-    dependent_begin();
+    dependent_begin<false>();
     const size_t row = blockIdx.x;
     const T *x = src + row * cols;
     T *y = dst + row * cols;
@@ -482,7 +482,7 @@ __global__ void add_kernel(T *__restrict__ dst, const T *__restrict__ a, const T
 template <typename T>
 __global__ void __launch_bounds__(256) add_vec_kernel(T *dst, const T *a, const T *b, size_t nvec) {
     constexpr int V = 16 / (int)sizeof(T);
-    dependent_begin();
+    dependent_begin<false>();
     const size_t i0 = (size_t)blockIdx.x * 512 + threadIdx.x;
     uint4 va[2], vb[2];
 #pragma unroll
@@ -1366,7 +1366,7 @@ int decode_attention_impl(void *out_bf16, const void *q_bf16, size_t q_batch_str
         XN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, decode_attention_combine_kernel, (__nv_bfloat16 *)out_bf16,
                                          (const float *)workspace, splits));
     }
-    if (x_hi) return xn_mm_split_rows_e4m3(x_hi, x_lo, x_scale, out_bf16, XN_BF16, batch, heads * head_dim, stream);
+    if (x_hi) return split_rows_e4m3(x_hi, x_lo, x_scale, out_bf16, XN_BF16, batch, heads * head_dim, true, stream);
     return XN_OK;
 }
 }  // namespace
@@ -1486,7 +1486,7 @@ extern "C" int xn_mm_decode_attention_append_e4m3(uint8_t *x_hi, uint8_t *x_lo, 
     cfg.blockDim = dim3(HD);
     XN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, decode_attention_combine_kernel, (__nv_bfloat16 *)out_bf16, (const float *)workspace,
                                      splits));
-    if (x_hi) return xn_mm_split_rows_e4m3(x_hi, x_lo, x_scale, out_bf16, XN_BF16, batch, heads * head_dim, stream);
+    if (x_hi) return split_rows_e4m3(x_hi, x_lo, x_scale, out_bf16, XN_BF16, batch, heads * head_dim, true, stream);
     return XN_OK;
 }
 

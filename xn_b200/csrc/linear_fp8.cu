@@ -101,7 +101,7 @@ extern "C" int xn_mm_linear_fp8(void *y_bf16, const void *x_bf16, const uint8_t 
     uint8_t *hi = (uint8_t *)workspace;
     uint8_t *lo = hi + round_up(m * k, 256);
     float *xs = (float *)(lo + round_up(m * k, 256));
-    int rc = xn_mm_split_rows_e4m3(hi, variant == 0 ? lo : nullptr, xs, x_bf16, XN_BF16, m, k, stream);
+    int rc = split_rows_e4m3(hi, variant == 0 ? lo : nullptr, xs, x_bf16, XN_BF16, m, k, true, stream);
     if (rc) return rc;
     return xn_mm_linear_fp8_pieces(y_bf16, hi, variant == 0 ? lo : nullptr, xs, wq, w_scale, m, n, k, stream);
 }
@@ -180,7 +180,7 @@ extern "C" int xn_mm_linear_fp8_noalloc(void *y_bf16, const void *x_bf16, const 
     uint8_t *hi = base;
     uint8_t *lo = base + NOALLOC_MAX_ELEMS;
     float *xs = reinterpret_cast<float *>(base + NOALLOC_SCALE_OFFSET);
-    rc = xn_mm_split_rows_e4m3(hi, variant == 0 ? lo : nullptr, xs, x_bf16, XN_BF16, m, k, stream);
+    rc = split_rows_e4m3(hi, variant == 0 ? lo : nullptr, xs, x_bf16, XN_BF16, m, k, true, stream);
     if (rc) return rc;
     // Up to 64 rows no kernel needs scratch of its own: the tensor-memory kernel's split tiles meet in shared memory.
     return xn_mm_linear_fp8_pieces(y_bf16, hi, variant == 0 ? lo : nullptr, xs, wq, w_scale, m, n, k, stream);

@@ -197,11 +197,11 @@ __global__ void split_rows_e4m3_kernel(uint8_t *__restrict__ x_hi, uint8_t *__re
 
 // Fast path of the split for 16-bit rows: 256 threads per row, each holds up to VPT 8-element vectors of
 // the row in registers between the maximum and the rounding pass (one read of x), 8-byte stores.
-template <typename T, int VPT>
+template <typename T, int VPT, bool EARLY>
 __global__ void __launch_bounds__(256)
 split_rows_e4m3_vec_kernel(uint8_t *x_hi, uint8_t *x_lo, float *x_scale, const T *x, size_t k) {
     __shared__ float red[32];
-    dependent_begin();
+    dependent_begin<EARLY>();
     const size_t row = blockIdx.x;
     const uint4 *src = reinterpret_cast<const uint4 *>(x + row * k);
     const int nvec = (int)(k / 8);
@@ -325,9 +325,10 @@ extern "C" int xn_mm_quantize_weights_fp8(uint8_t *wq, float *w_scale, const voi
     return XN_OK;
 }
 
-extern "C" int xn_mm_split_rows_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_scale, const void *x,
-                                     xn_dtype dtype, size_t m, size_t k, void *stream) {
-    XN_API_RANGE("xn_mm_split_rows_e4m3");
+// `pieces_only`: the pieces are this library's own activations, so the next kernel may begin early; a caller's pieces have
+// the layout of an fp8 weight and may be used as one (see dependent_begin).
+int xn::split_rows_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_scale, const void *x, xn_dtype dtype, size_t m, size_t k, bool pieces_only,
+                        void *stream) {
     XN_REQUIRE(valid_dtype(dtype), "split_rows_e4m3: unknown dtype %d", (int)dtype);
     if (m == 0 || k == 0) return XN_OK;
     XN_REQUIRE(x_hi && x_scale && x, "split_rows_e4m3: null pointer");
@@ -338,7 +339,8 @@ extern "C" int xn_mm_split_rows_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_scal
         const bool small = k <= 8 * 256 * 2;
         auto go = [&](auto *p) {
             using T = std::remove_const_t<std::remove_pointer_t<decltype(p)>>;
-            auto kern = small ? split_rows_e4m3_vec_kernel<T, 2> : split_rows_e4m3_vec_kernel<T, 8>;
+            auto kern = pieces_only ? (small ? split_rows_e4m3_vec_kernel<T, 2, true> : split_rows_e4m3_vec_kernel<T, 8, true>)
+                                    : (small ? split_rows_e4m3_vec_kernel<T, 2, false> : split_rows_e4m3_vec_kernel<T, 8, false>);
             return launch_dependent(kern, dim3((unsigned)m), dim3(256), 0, st, x_hi, x_lo, x_scale, p, k);
         };
         return dtype == XN_BF16 ? go((const __nv_bfloat16 *)x) : go((const __half *)x);
@@ -347,4 +349,10 @@ extern "C" int xn_mm_split_rows_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_scal
         split_rows_e4m3_kernel<T><<<(unsigned)m, 256, 0, st>>>(x_hi, x_lo, x_scale, (const T *)x, k));
     XN_CHECK_CUDA(cudaGetLastError());
     return XN_OK;
+}
+
+extern "C" int xn_mm_split_rows_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_scale, const void *x, xn_dtype dtype, size_t m, size_t k,
+                                     void *stream) {
+    XN_API_RANGE("xn_mm_split_rows_e4m3");
+    return xn::split_rows_e4m3(x_hi, x_lo, x_scale, x, dtype, m, k, false, stream);
 }
