@@ -368,35 +368,33 @@ __device__ __forceinline__ void pack_store(T *row, int cin, int c, T v) {
     }
 }
 
-// xt[b][lead + l][c] = x[b][c][l]; rows outside [lead, lead + length) are zero.  32 x 32 tiles through
-// shared memory so that both the reads (along l) and the writes (along c) are coalesced.
+// xt[b][lead + l][c] = x[b][c][l]; rows outside [lead, lead + length) are zero.  32 positions x 128 channels per block
+// through shared memory, so that both the reads (along l) and the writes (along c) are coalesced.
 constexpr int PI_C = 128;   // channels per block of the input repack
 template <typename T>
-__global__ void __launch_bounds__(256)
-conv_pack_input_kernel(T *__restrict__ xt, const T *__restrict__ x, int cin, int length, int lead, int rows) {
-    // 32 positions x 128 channels per block: 16 independent loads per thread in flight, output rows written in
-    // runs of 128 channels
-    __shared__ T tile[PI_C][33];
-    const int b = blockIdx.z, r0 = blockIdx.x * 32, c0 = blockIdx.y * PI_C;
+__device__ __forceinline__ void pack_input_block(T *xt, const T *x, T *tile, int cin, int length, int lead, int rows, int b, int r0, int c0) {
+    constexpr int PITCH = 33;
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     const T *xb = x + (size_t)b * cin * length;
     T *xtb = xt + (size_t)b * rows * cin * pack_mult<T>();
     const int l = r0 + tx - lead;
     const bool lok = l >= 0 && l < length;
-#pragma unroll 8
-    for (int i = ty; i < PI_C; i += 8) {
-        const int c = c0 + i;
-        T v = from_f32<T>(0.f);
-        if (lok && c < cin) v = xb[(size_t)c * length + l];
-        tile[i][tx] = v;
+    T v[PI_C / 8];
+#pragma unroll
+    for (int i = 0; i < PI_C / 8; ++i) {
+        const int c = c0 + ty + 8 * i;
+        v[i] = from_f32<T>(0.f);
+        if (lok && c < cin) v[i] = ld_act(xb + (size_t)c * length + l);
     }
+#pragma unroll
+    for (int i = 0; i < PI_C / 8; ++i) tile[(ty + 8 * i) * PITCH + tx] = v[i];
     __syncthreads();
     const int c = threadIdx.x & (PI_C - 1);
     if (c0 + c < cin) {
 #pragma unroll 4
         for (int i = threadIdx.x / PI_C; i < 32; i += 256 / PI_C) {
             const int r = r0 + i;
-            if (r < rows) pack_store<T, false>(xtb + (size_t)r * cin * pack_mult<T>(), cin, c0 + c, tile[c][i]);
+            if (r < rows) pack_store<T, false>(xtb + (size_t)r * cin * pack_mult<T>(), cin, c0 + c, tile[c * PITCH + i]);
         }
     }
 }
@@ -441,17 +439,15 @@ conv_pack_taps_tr_kernel(T *__restrict__ wp, const T *__restrict__ w, int cin, i
 // ((r * cout + co) * taps + j) holding tap kk = r + stride * (taps - 1 - j) or zeros.
 constexpr int PK_CC = 64;
 template <typename T, bool TR>
-__global__ void __launch_bounds__(256)
-conv_pack_taps_tiled_kernel(T *__restrict__ wp, const T *__restrict__ w, int cin, int cout, int ksize, int stride, int taps) {
-    extern __shared__ __align__(16) unsigned char pk_smem[];
-    T *tile = reinterpret_cast<T *>(pk_smem);   // [PK_CC][ksize + 1]
-    const int co = blockIdx.x, c0 = blockIdx.y * PK_CC, pitch = ksize + 1;
+__device__ __forceinline__ void pack_taps_block(T *wp, const T *w, T *tile, int cin, int cout, int ksize, int stride, int taps, int co, int c0) {
+    const int pitch = ksize + 1;  // tile: [PK_CC][pitch]
     const size_t ci_stride = TR ? (size_t)cout * ksize : (size_t)ksize;
     const T *base = TR ? w + (size_t)co * ksize : w + (size_t)co * cin * ksize;
+#pragma unroll 4
     for (int e = threadIdx.x; e < PK_CC * ksize; e += 256) {
-        const int ci = e / ksize, kk = e - ci * ksize;
+        const int ci = (int)((unsigned)e / (unsigned)ksize), kk = e - ci * ksize;
         T v = from_f32<T>(0.f);
-        if (c0 + ci < cin) v = base[(size_t)(c0 + ci) * ci_stride + kk];
+        if (c0 + ci < cin) v = ld_act(base + (size_t)(c0 + ci) * ci_stride + kk);
         tile[ci * pitch + kk] = v;
     }
     __syncthreads();
@@ -473,26 +469,48 @@ conv_pack_taps_tiled_kernel(T *__restrict__ wp, const T *__restrict__ w, int cin
     }
 }
 
+// Both repackings in one launch: the blocks that move taps first, then the input's.  A streaming step is a chain of
+// launches of a few microseconds each, so what there is to save is one launch, and the start of the next (every kernel of
+// the chain is launched dependent): f32 512 -> 512 channels, 7 taps, 64 positions 27.7 -> 22.0 us.
+template <typename T, bool TR>
+__global__ void __launch_bounds__(256)
+conv_pack_kernel(T *xt, T *wp, const T *x, const T *w, int cin, int cout, int length, int lead, int rows, int ksize, int stride, int taps,
+                 unsigned tap_blocks, unsigned tap_chunks, unsigned row_blocks, unsigned channel_blocks) {
+    extern __shared__ __align__(16) unsigned char pk_smem[];
+    T *tile = reinterpret_cast<T *>(pk_smem);
+    dependent_begin();
+    unsigned i = blockIdx.x;
+    if (i < tap_blocks) {
+        const unsigned co = i / tap_chunks, cc = i - co * tap_chunks;
+        pack_taps_block<T, TR>(wp, w, tile, cin, cout, ksize, stride, taps, (int)co, (int)cc * PK_CC);
+    } else {
+        i -= tap_blocks;
+        const unsigned rb = i % row_blocks, t = i / row_blocks, cb = t % channel_blocks, b = t / channel_blocks;
+        pack_input_block<T>(xt, x, tile, cin, length, lead, rows, (int)b, (int)rb * 32, (int)cb * PI_C);
+    }
+}
+
 // Phase interleave through shared memory: one block per (batch entry, out channel, 512 values of q); rows of d
 // are read contiguously, the output run of 512 * stride positions is written contiguously.
 constexpr int IL_QT = 512;
 template <typename T>
 __global__ void __launch_bounds__(256)
-conv_interleave_tiled_kernel(T *__restrict__ out, const T *__restrict__ d, const T *__restrict__ bias, int cout, int out_length,
+conv_interleave_tiled_kernel(T *out, const T *d, const T *bias, int cout, int out_length,
                              int stride, int padding, int nq) {
     extern __shared__ __align__(16) unsigned char il_smem[];
     T *tile = reinterpret_cast<T *>(il_smem);
     constexpr int PITCH = IL_QT + 4 / (int)sizeof(T);   // an odd number of 32-bit words: phases fall in distinct banks
+    dependent_begin<false>();
     const int q0 = blockIdx.x * IL_QT, co = blockIdx.y, b = blockIdx.z;
     const T *db = d + ((size_t)b * stride * cout + co) * nq;
     const size_t row_pitch = (size_t)cout * nq;
 #pragma unroll 4
     for (int i = threadIdx.x; i < stride * IL_QT; i += 256) {
         const int r = i / IL_QT, q = i - r * IL_QT;
-        if (q0 + q < nq) tile[r * PITCH + q] = db[r * row_pitch + q0 + q];
+        if (q0 + q < nq) tile[r * PITCH + q] = ld_act(db + r * row_pitch + q0 + q);
     }
     __syncthreads();
-    const float bv = bias ? to_f32(bias[co]) : 0.f;
+    const float bv = bias ? to_f32(ld_act(bias + co)) : 0.f;
     T *ob = out + ((size_t)b * cout + co) * out_length;
     // output position q0 * stride + i - padding holds (q, r) = (i / stride, i % stride); i advances by 256 per
     // iteration, so (q, r) advance by (256 / stride, 256 % stride) with a carry: one division per thread
@@ -526,14 +544,20 @@ conv_interleave_kernel(T *__restrict__ out, const T *__restrict__ d, const T *__
     }
 }
 
-// out[row][col] = sum over splits of part[s][row][col] (+ bias[row]), summed in split order
+// out[row][col] = sum over splits of part[s][row][col] (+ bias[row]), summed in split order; four loads in flight per thread
 __global__ void __launch_bounds__(256)
-conv_sum_partials_kernel(float *__restrict__ out, const float *__restrict__ part, const float *__restrict__ bias, int splits,
-                         size_t n, size_t total) {
+conv_sum_partials_kernel(float *out, const float *part, const float *bias, int splits, size_t n, size_t total) {
+    dependent_begin<false>();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         float s = 0.f;
-        for (int k = 0; k < splits; ++k) s += part[(size_t)k * total + i];
-        if (bias) s += bias[i / n];
+        for (int k = 0; k < splits; k += 4) {
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = k + j < splits ? ld_act_f32(part + (size_t)(k + j) * total + i) : 0.f;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) s += v[j];
+        }
+        if (bias) s += ld_act_f32(bias + i / n);
         out[i] = s;
     }
 }
@@ -603,20 +627,26 @@ int launch_conv_gemm(xn_dtype dt, T *dst, const T *src, const T *kernel, const T
     T *wp = reinterpret_cast<T *>(ws + p.xt_bytes);
     T *d = reinterpret_cast<T *>(ws + p.xt_bytes + p.wp_bytes);
     const int lead = TR ? p.taps - 1 : a.padding;
-    dim3 pg((unsigned)((p.rows + 31) / 32), (unsigned)((cin + PI_C - 1) / PI_C), (unsigned)a.batch);
-    conv_pack_input_kernel<T><<<pg, 256, 0, st>>>(xt, src, cin, a.length, lead, p.rows);
     const size_t wtotal = TR ? (size_t)a.stride * cout * p.taps * cin : (size_t)cout * a.ksize * cin;
-    const unsigned wgrid = (unsigned)((wtotal + 255) / 256 < 4096 ? (wtotal + 255) / 256 : 4096);
-    const size_t pk_smem = (size_t)PK_CC * (a.ksize + 1) * sizeof(T);
-    if (pk_smem <= 40 * 1024 && cout <= 0x7fffffff / 2 && (cin + PK_CC - 1) / PK_CC <= 65535) {
-        dim3 wg((unsigned)cout, (unsigned)((cin + PK_CC - 1) / PK_CC));
-        conv_pack_taps_tiled_kernel<T, TR><<<wg, 256, pk_smem, st>>>(wp, kernel, cin, cout, a.ksize, a.stride, p.taps);
-    } else if (!TR) {
-        conv_pack_taps_kernel<T><<<wgrid, 256, 0, st>>>(wp, kernel, cin, a.ksize, wtotal);
-    } else {
-        conv_pack_taps_tr_kernel<T><<<wgrid, 256, 0, st>>>(wp, kernel, cin, cout, a.ksize, a.stride, p.taps, wtotal);
+    const size_t pk_smem = (size_t)PK_CC * (a.ksize + 1) * sizeof(T), in_smem = (size_t)PI_C * 33 * sizeof(T);
+    // blocks that repack the taps (none when their tile does not fit: then the per-element kernels do it) and the input
+    const bool tiled_taps = pk_smem <= 40 * 1024;
+    const size_t tap_chunks = (size_t)(cin + PK_CC - 1) / PK_CC, tap_blocks = tiled_taps ? (size_t)cout * tap_chunks : 0;
+    const size_t row_blocks = (size_t)(p.rows + 31) / 32, channel_blocks = (size_t)(cin + PI_C - 1) / PI_C;
+    const size_t blocks_all = tap_blocks + row_blocks * channel_blocks * (size_t)a.batch;
+    XN_REQUIRE(blocks_all <= 0x7fffffff, "conv: too many blocks in the repacking launch");
+    const size_t smem = tiled_taps && pk_smem > in_smem ? pk_smem : in_smem;
+    XN_ENSURE_SMEM((conv_pack_kernel<T, TR>), smem);
+    if (int rc = launch_dependent(conv_pack_kernel<T, TR>, dim3((unsigned)blocks_all), dim3(256), smem, st, xt, wp, src, kernel, cin, cout,
+                                  a.length, lead, p.rows, a.ksize, a.stride, p.taps, (unsigned)tap_blocks, (unsigned)tap_chunks,
+                                  (unsigned)row_blocks, (unsigned)channel_blocks))
+        return rc;
+    if (!tiled_taps) {
+        const unsigned wgrid = (unsigned)((wtotal + 255) / 256 < 4096 ? (wtotal + 255) / 256 : 4096);
+        if (!TR) conv_pack_taps_kernel<T><<<wgrid, 256, 0, st>>>(wp, kernel, cin, a.ksize, wtotal);
+        else conv_pack_taps_tr_kernel<T><<<wgrid, 256, 0, st>>>(wp, kernel, cin, cout, a.ksize, a.stride, p.taps, wtotal);
+        XN_CHECK_CUDA(cudaGetLastError());
     }
-    XN_CHECK_CUDA(cudaGetLastError());
     const size_t cpr = (size_t)cin * pack_mult<T>();   // packed row length
     const size_t k = (size_t)p.taps * cpr;
     auto gemm = [&](T *out, const T *row_bias, size_t m, size_t n, size_t ldb, size_t out_bs) -> int {
@@ -626,9 +656,7 @@ int launch_conv_gemm(xn_dtype dt, T *dst, const T *src, const T *kernel, const T
                 if (int rc = launch_gemm_tn_tf32_splitk(part, wp, xt, m, n, k / p.splits, p.splits, k, ldb, st)) return rc;
                 const size_t total = m * n;
                 const unsigned grid = (unsigned)((total + 255) / 256 < 2048 ? (total + 255) / 256 : 2048);
-                conv_sum_partials_kernel<<<grid, 256, 0, st>>>(out, part, row_bias, p.splits, n, total);
-                XN_CHECK_CUDA(cudaGetLastError());
-                return XN_OK;
+                return launch_dependent(conv_sum_partials_kernel, dim3(grid), dim3(256), 0, st, out, part, row_bias, p.splits, n, total);
             }
             return launch_gemm_tn_tf32_shared_lhs(out, wp, xt, row_bias, m, n, k, k, ldb, n, a.batch, (size_t)p.rows * cpr, out_bs, st);
         } else
@@ -644,7 +672,8 @@ int launch_conv_gemm(xn_dtype dt, T *dst, const T *src, const T *kernel, const T
     const size_t il_smem = (size_t)a.stride * (IL_QT + 4 / sizeof(T)) * sizeof(T);
     if (il_smem <= 40 * 1024 && cout <= 65535) {
         dim3 ig((unsigned)((p.nq + IL_QT - 1) / IL_QT), (unsigned)cout, (unsigned)a.batch);
-        conv_interleave_tiled_kernel<T><<<ig, 256, il_smem, st>>>(dst, d, bias, cout, a.out_length, a.stride, a.padding, p.nq);
+        return launch_dependent(conv_interleave_tiled_kernel<T>, ig, dim3(256), il_smem, st, dst, d, bias, cout, a.out_length, a.stride,
+                                a.padding, p.nq);
     } else {
         conv_interleave_kernel<T><<<grid, 256, 0, st>>>(dst, d, bias, cout, a.out_length, a.stride, a.padding, p.nq, total);
     }
