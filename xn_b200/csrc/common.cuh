@@ -233,7 +233,9 @@ int launch_attention_prefill(xn_dtype dt, void *out, size_t ldo, const void *q, 
                              size_t head_stride, size_t heads, size_t t_rows, size_t ctx, float scale, cudaStream_t st);
 // runtime.cu: library-owned scratch per (device, stream) and the device status word
 struct SkinnyScratch { float *partials = nullptr; size_t partial_bytes = 0; unsigned *counters = nullptr; size_t ncounters = 0; };
-int skinny_scratch(cudaStream_t st, size_t partial_bytes, size_t ncounters, SkinnyScratch *out);
+constexpr int SCRATCH_MAIN = 0;  // operands repacked for a launch, split sums
+constexpr int SCRATCH_TAIL = 1;  // the tiled kernel's records of cut tiles: its operands may lie in the other buffer
+int skinny_scratch(cudaStream_t st, size_t partial_bytes, size_t ncounters, SkinnyScratch *out, int slot = SCRATCH_MAIN);
 int library_scratch(cudaStream_t st, size_t bytes, void **out);
 struct WaitCtx;
 // Fills the bound and the status-word pointer every kernel with device-side waits takes; fails with

@@ -76,8 +76,11 @@ struct GemmArgs {
     int rows2;            // NA = 2 instantiations: the two A tiles are rows [256 i, +128) and [256 i + 128, +128) of ONE matrix
                           // (a 256 x BN tile: both accumulator buffers belong to one tile, the B stage is read by two MMAs)
     int fast_store;       // one destination, no multicast, and every 16-byte output chunk of an interior tile is aligned
-    float *split_out;     // split-k launch: the batch index is a k chunk of ONE product and every tile leaves as an f32
-                          // record [chunk][tile][column group of 4][128 rows][4] for splitk_reduce_kernel
+    // The last, partly filled round (see tail_parts): tiles from full_tiles on are cut into tail_split ranges of k, each a unit
+    // of its own that leaves as an f32 record [tile][accumulator][range][column group of 4][128 rows][4] in tail_rec for
+    // tail_reduce_kernel.  tail_split <= 1: no tile is cut.
+    int full_tiles, tail_split;
+    float *tail_rec;
 };
 
 __device__ __forceinline__ bool tile_masked(const GemmArgs &a, int m_blk, int n_blk, int bn) {
@@ -90,6 +93,28 @@ __device__ __forceinline__ int tile_kb(const GemmArgs &a, int m_blk, int num_kb,
     return kb < 1 ? 1 : min(kb, num_kb);
 }
 
+// What a CTA does for index v of its round-robin: a whole tile, or (part >= 0) one range of k of a tile of the last round.
+struct Unit { int tile, kb0, kb1, part; };
+__device__ __forceinline__ Unit unit_of(const GemmArgs &a, int v, int num_tiles, int num_kb) {
+    if (a.tail_split <= 1 || v < a.full_tiles) return {v, 0, num_kb, -1};
+    const int tail = num_tiles - a.full_tiles, u = v - a.full_tiles, part = u / tail;
+    return {a.full_tiles + (u - part * tail), num_kb * part / a.tail_split, num_kb * (part + 1) / a.tail_split, part};
+}
+// One warp's share of a tile's accumulators (lane quarter q, 32-column chunks [c_begin, c_end)) as an f32 record: a lane's
+// row of every 4-column group next to its neighbours' rows, 512 contiguous bytes per warp access.
+__device__ __forceinline__ void store_record(float *rec, uint32_t lane_addr, int q, int lane, int c_begin, int c_end) {
+    rec += (size_t)(q * 32 + lane) * 4;
+#pragma unroll 1
+    for (int c = c_begin; c < c_end; ++c) {
+        uint32_t v[32];
+        tmem_ld32(lane_addr + c * 32, v);
+#pragma unroll
+        for (int j4 = 0; j4 < 8; ++j4)
+            *reinterpret_cast<float4 *>(rec + (size_t)(c * 8 + j4) * (BM * 4)) =
+                make_float4(__uint_as_float(v[4 * j4]), __uint_as_float(v[4 * j4 + 1]), __uint_as_float(v[4 * j4 + 2]),
+                            __uint_as_float(v[4 * j4 + 3]));
+    }
+}
 // Epilogue of one output tile for the fp8 / bf16 / f16 kinds.  Eight warps share a tile: warp (q, half) owns the
 // 32 accumulator rows of tensor-memory lane quarter q (output rows m_row0 + 32 q ..) and the 32-column chunks
 // [c_begin, c_end) of buffer `acc`.  Two chunks at a time are loaded together, scaled / biased, rounded to the
@@ -103,25 +128,6 @@ template <int KIND, int BN>
 __device__ __forceinline__ void epilogue_tile(const GemmArgs &args, uint32_t tmem_base, int acc, int q, int lane, int m_row0,
                                               int n_blk, int g, unsigned char *slab, int c_begin, int c_end) {
     constexpr bool F8 = KIND == 0;
-    if (args.split_out) {
-        // raw f32 accumulators, a lane's row of every 4-column group next to its neighbours' rows: 512 contiguous
-        // bytes per warp store; scales, bias and rounding belong to the reduction over the chunks
-        const int num_n = (args.N + BN - 1) / BN, num_m = (args.M + BM - 1) / BM;
-        const size_t t = (size_t)g * num_m * num_n + (size_t)(m_row0 / BM) * num_n + n_blk;
-        float *rec = args.split_out + t * (size_t)(BN * BM) + (size_t)(q * 32 + lane) * 4;
-        const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BN);
-#pragma unroll 1
-        for (int c = c_begin; c < c_end; ++c) {
-            uint32_t v[32];
-            tmem_ld32(taddr + c * 32, v);
-#pragma unroll
-            for (int j4 = 0; j4 < 8; ++j4)
-                *reinterpret_cast<float4 *>(rec + (size_t)(c * 8 + j4) * (BM * 4)) =
-                    make_float4(__uint_as_float(v[4 * j4]), __uint_as_float(v[4 * j4 + 1]), __uint_as_float(v[4 * j4 + 2]),
-                                __uint_as_float(v[4 * j4 + 3]));
-        }
-        return;
-    }
     const int row = m_row0 + q * 32 + lane;
     float xs = 1.0f;
     if (F8 && row < args.M) xs = ld_act_f32(args.x_scale + row);
@@ -289,6 +295,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
     const int tiles_per_batch = num_m * num_n;
     const int num_tiles = tiles_per_batch * args.batch;
     const int num_kb = (args.K + BK - 1) / BK;
+    const int num_units = KIND != 3 && args.tail_split > 1 ? args.full_tiles + (num_tiles - args.full_tiles) * args.tail_split : num_tiles;
 
     if (threadIdx.x == 0) {
         prefetch_tmap(&map_a0);
@@ -319,13 +326,14 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
         if (elect_one()) {
             int it = 0;  // running k-block count across tiles: stage = it % NSTAGE
             bool ok = true;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-                const int g = tile / tiles_per_batch, tin = tile % tiles_per_batch;
+            for (int v = blockIdx.x; v < num_units && ok; v += gridDim.x) {
+                const Unit unit = KIND == 3 ? Unit{v, 0, num_kb, -1} : unit_of(args, v, num_tiles, num_kb);
+                const int g = unit.tile / tiles_per_batch, tin = unit.tile % tiles_per_batch;
                 int m_blk, n_blk;
                 tile_coords(tin, num_m, num_n, args.group_m, m_blk, n_blk);
                 if (KIND != 3 && tile_masked(args, m_blk, n_blk, BN)) continue;
-                const int nkb = KIND != 3 ? tile_kb(args, m_blk, num_kb, BK) : num_kb;
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
+                const int kb_end = KIND != 3 ? tile_kb(args, m_blk, unit.kb1, BK) : unit.kb1;
+                for (int kb = unit.kb0; kb < kb_end; ++kb, ++it) {
                     const int s = it % NSTAGE;
                     const unsigned ph = (unsigned)(it / NSTAGE) & 1u;
                     if (!mbar_wait(&empty[s], ph ^ 1u, args.wait)) { ok = false; break; }
@@ -356,11 +364,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
         if (elect_one()) {
             int it = 0, vt = 0;   // vt: accumulator hand-overs to the epilogue so far (one per tile, or per k chunk)
             bool ok = true;
-            for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-            int nkb = num_kb;
+            for (int v = blockIdx.x; v < num_units && ok; v += gridDim.x) {
+            const Unit unit = KIND == 3 ? Unit{v, 0, num_kb, -1} : unit_of(args, v, num_tiles, num_kb);
+            int nkb = unit.kb1 - unit.kb0;
             if (KIND != 3 && args.causal) {
                 int m_blk, n_blk;
-                tile_coords(tile % tiles_per_batch, num_m, num_n, args.group_m, m_blk, n_blk);
+                tile_coords(unit.tile % tiles_per_batch, num_m, num_n, args.group_m, m_blk, n_blk);
                 if (tile_masked(args, m_blk, n_blk, BN)) continue;
                 nkb = tile_kb(args, m_blk, num_kb, BK);
             }
@@ -497,8 +506,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
                 }
             }
         } else
-        for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-            const int g = tile / tiles_per_batch, tin = tile % tiles_per_batch;
+        for (int v = blockIdx.x; v < num_units && ok; v += gridDim.x) {
+            const Unit unit = KIND == 3 ? Unit{v, 0, num_kb, -1} : unit_of(args, v, num_tiles, num_kb);
+            const int g = unit.tile / tiles_per_batch, tin = unit.tile % tiles_per_batch;
             int m_blk, n_blk;
             tile_coords(tin, num_m, num_n, args.group_m, m_blk, n_blk);
             if (tile_masked(args, m_blk, n_blk, BN)) continue;
@@ -509,12 +519,19 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_con
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // warps 2-5 take the first half of the tile's 32-column chunks, warps 6-9 the second (odd counts: one more first)
             constexpr int NCHUNK = BN / 32, FIRST = (NCHUNK + 1) / 2;
-            const int half = (warp - 2) >> 2;
-            epilogue_tile<KIND, BN>(args, tmem_base, acc, q, lane, m_blk * BMT, n_blk, g, epi_smem + (size_t)(warp - 2) * 4096,
-                                    half ? FIRST : 0, half ? NCHUNK : FIRST);
-            if (rows2)  // rows 128..255 of the tile sit in the second buffer
-                epilogue_tile<KIND, BN>(args, tmem_base, 1, q, lane, m_blk * BMT + BM, n_blk, g, epi_smem + (size_t)(warp - 2) * 4096,
-                                        half ? FIRST : 0, half ? NCHUNK : FIRST);
+            const int half = (warp - 2) >> 2, c_begin = half ? FIRST : 0, c_end = half ? NCHUNK : FIRST;
+            unsigned char *slab = epi_smem + (size_t)(warp - 2) * 4096;
+            // rows2: rows 128..255 of the tile sit in the second buffer
+            for (int a = 0; a < (rows2 ? 2 : 1); ++a) {
+                const int buf = rows2 ? a : acc;
+                if (unit.part >= 0) {  // one range of k of a tile of the last round
+                    const int at = (unit.tile - args.full_tiles) * (rows2 ? 2 : 1) + a;
+                    store_record(args.tail_rec + ((size_t)at * args.tail_split + unit.part) * (BN * BM),
+                                 tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * BN), q, lane, c_begin, c_end);
+                } else {
+                    epilogue_tile<KIND, BN>(args, tmem_base, buf, q, lane, m_blk * BMT + a * BM, n_blk, g, slab, c_begin, c_end);
+                }
+            }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
             if (lane == 0) mbar_arrive(&tmem_empty[acc]);
@@ -1065,30 +1082,37 @@ attention_prefill_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 }
 
 // ---- host side ----
-// Second half of a split-k product: y = epilogue(sum over the k chunks of the f32 tile records the tiled kernel left
-// in `rec`), the chunks added in k order.  A thread owns one row of a tile and one group of 4 columns; a CTA of 256
-// threads covers the tile's 128 rows x 2 column groups, so every record read is 512 contiguous bytes per warp.
-// Epilogue as in the tiled kernel: fp8 scales, or nn::Linear's bias added to the rounded product and rounded again.
+// Second half of the tiles that were cut along k: y = epilogue(sum over the ranges of the f32 records the tiled kernel left
+// in tail_rec), added in k order.  A thread owns one row of a tile and one group of 4 columns; a CTA of 256 threads covers
+// 128 rows x 2 column groups, so every record read is 512 contiguous bytes per warp.  Epilogue as in the tiled kernel: fp8
+// scales, or nn::Linear's bias added to the rounded product and rounded again.  A launch of its own because the sum is
+// wanted from the whole machine: the form in which the last CTA to arrive at a tile added its records read 4 x 128 KB
+// through one SM (bf16 1024 x 5120 x 4096: 47.2 us, 42.6 with this kernel, 39.5 without any cut; f16 3001 x
+// 4096 x 11264: 207 and 202.5 us).  Split-k of a product with few tiles is the same thing with no full round, so the launch
+// pair that did only that is gone: bf16 300 x 4096 x 8192 47.5 -> 32.3 us, W8A16 200 x 4096 x 4096 26.4 -> 20 us (narrow tiles).
 template <int KIND>
 __global__ void __launch_bounds__(256)
-splitk_reduce_kernel(void *__restrict__ y, int ldy, const float *__restrict__ rec, int chunks, int M, int N, int bn,
-                     const float *__restrict__ x_scale, const float *__restrict__ w_scale, const void *__restrict__ col_bias) {
+tail_reduce_kernel(const GemmArgs args, int bn, int nacc, int tiles_per_batch, int num_m, int num_n) {
     constexpr bool F8 = KIND == 0;
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int per_tile = bn / 8;  // CTAs per tile
-    const int t = blockIdx.x / per_tile, cg = (blockIdx.x - t * per_tile) * 2 + (threadIdx.x >> 7), r = threadIdx.x & 127;
-    const int num_n = (N + bn - 1) / bn, num_m = (M + BM - 1) / BM;
-    const int m_blk = t / num_n, n_blk = t - m_blk * num_n;
-    const int row = m_blk * BM + r, col = n_blk * bn + cg * 4;
-    if (row >= M || col >= N) return;
-    const size_t tile_elems = (size_t)bn * BM, chunk_elems = tile_elems * num_m * num_n;
-    const float *p = rec + (size_t)t * tile_elems + ((size_t)cg * BM + r) * 4;
+    const int per_tile = bn / 8;  // CTAs per accumulator
+    const int at = blockIdx.x / per_tile, cg = (blockIdx.x - at * per_tile) * 2 + (threadIdx.x >> 7), r = threadIdx.x & 127;
+    const int t = at / nacc, tile = args.full_tiles + t, g = tile / tiles_per_batch;
+    int m_blk, n_blk;
+    tile_coords(tile - g * tiles_per_batch, num_m, num_n, args.group_m, m_blk, n_blk);
+    const int row = (m_blk * nacc + (at - t * nacc)) * BM + r, col = n_blk * bn + cg * 4;
+    if (row >= args.M || col >= args.N) return;
+    const int N = args.N, ldy = args.ldy, chunks = args.tail_split;
+    const float *x_scale = args.x_scale, *w_scale = args.w_scale;
+    const void *col_bias = args.col_bias;
+    const size_t rec_elems = (size_t)bn * BM;
+    const float *p = args.tail_rec + (size_t)at * chunks * rec_elems + ((size_t)cg * BM + r) * 4;
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int c0 = 0; c0 < chunks; c0 += 4) {
         float4 v[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j)
-            v[j] = c0 + j < chunks ? __ldcg(reinterpret_cast<const float4 *>(p + (size_t)(c0 + j) * chunk_elems))
+            v[j] = c0 + j < chunks ? __ldcg(reinterpret_cast<const float4 *>(p + (size_t)(c0 + j) * rec_elems))
                                    : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int j = 0; j < 4; ++j) { sum.x += v[j].x; sum.y += v[j].y; sum.z += v[j].z; sum.w += v[j].w; }
@@ -1113,7 +1137,7 @@ splitk_reduce_kernel(void *__restrict__ y, int ldy, const float *__restrict__ re
             out[e] = *reinterpret_cast<const uint16_t *>(&h);
         }
     }
-    uint16_t *dst = reinterpret_cast<uint16_t *>(y) + (size_t)row * ldy + col;
+    uint16_t *dst = reinterpret_cast<uint16_t *>(args.y[0]) + (size_t)g * args.y_batch_stride + (size_t)row * ldy + args.col_offset + col;
     if (col + 4 <= N && (reinterpret_cast<uintptr_t>(dst) & 7) == 0) {
         *reinterpret_cast<uint2 *>(dst) = make_uint2((uint32_t)out[0] | ((uint32_t)out[1] << 16), (uint32_t)out[2] | ((uint32_t)out[3] << 16));
     } else {
@@ -1122,6 +1146,36 @@ splitk_reduce_kernel(void *__restrict__ y, int ldy, const float *__restrict__ re
 }
 
 struct BatchGeom { size_t batch = 1, a_stride = 0, b_stride = 0; };
+
+// A launch lasts as many rounds of tiles as the busiest SM gets, and the last round is rarely full.  When it fills at most
+// half of the SMs its tiles are cut along k into `parts` ranges that run side by side.  The price is an f32 record per
+// range written and read back through L2 and a launch that adds them: about 13 us at 128 x 256 tiles, tail_stages() k
+// stages.  us, no cut / cut: f16 3001 x 4096 x 11264 (192 tiles of 256 x 256: 148 + 44, three ranges) 230 / 202.5; bf16
+// 300 x 4096 x 8192 34.7 / 32.3; fp8 W8A16 4096 x 4096 x 11264 300 / 288.  Where the line is too low: bf16 1024 x 5120 x 4096
+// (64 stages) 39.5 / 42.6 at 24, 512 x 4096 x 4096 20.2 / 27.4 at 8; more than four ranges add records, not speed.
+constexpr int TAIL_MAX_PARTS = 4;
+constexpr int TAIL_MIN_STAGES = 8;  // k stages per range
+constexpr int tail_stages(int na) { return na == 2 ? 16 : 32; }  // a stage of two A tiles takes about twice as long
+inline int tail_parts(long long tiles, int num_kb, int na) {
+    const long long sms = sm_count(), tail = tiles % sms;
+    if (tail == 0 || tail * 2 > sms) return 1;
+    long long parts = sms / tail < TAIL_MAX_PARTS ? sms / tail : TAIL_MAX_PARTS;
+    if (parts > num_kb / TAIL_MIN_STAGES) parts = num_kb / TAIL_MIN_STAGES;
+    return parts > 1 && num_kb - num_kb / parts > tail_stages(na) ? (int)parts : 1;
+}
+// Rounds of whole tiles the launch lasts.
+inline double tile_rounds(long long tiles, int num_kb, int na, bool may_cut) {
+    const long long sms = sm_count(), parts = may_cut ? tail_parts(tiles, num_kb, na) : 1;
+    if (parts <= 1) return (double)((tiles + sms - 1) / sms);
+    return (double)(tiles / sms) + 1.0 / (double)parts + (double)tail_stages(na) / num_kb;
+}
+// A captured launch may be replayed beside anything: it takes no scratch it would share.  Peers' buffers and the
+// convolutions' row bias stay with the tiled kernel's own epilogue.
+inline bool may_cut_tail(const GemmArgs &a, cudaStream_t st) {
+    if (a.causal || a.ndst != 1 || a.mc || a.row_bias) return false;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
 
 template <int KIND, int BN, int NA>
 int launch_cfg(const void *a0, const void *a1, const void *b, size_t lda, size_t ldb, const GemmArgs &args,
@@ -1169,7 +1223,23 @@ int launch_cfg(const void *a0, const void *a1, const void *b, size_t lda, size_t
     const int bmt_rows = (NA == 2 && args.rows2) ? 2 * BM : BM;
     const long long tiles = (long long)((args.M + bmt_rows - 1) / bmt_rows) * ((args.N + BN - 1) / BN) * args.batch;
     const int sms = sm_count();
-    const int grid = (int)(tiles < sms ? tiles : sms);
+    long long units = tiles;
+    args2.tail_split = 1;
+    const int nacc = NA == 2 && args.rows2 ? 2 : 1;
+    const size_t tail = (size_t)(tiles % sms) * nacc;
+    if (KIND != 3 && may_cut_tail(args, st)) {
+        const int parts = tail_parts(tiles, (args.K + BKB / ELEM - 1) / (BKB / ELEM), NA);
+        SkinnyScratch sc;
+        if (parts > 1 && skinny_scratch(st, tail * parts * BN * BM * sizeof(float), 0, &sc, SCRATCH_TAIL) == XN_OK) {
+            args2.full_tiles = (int)(tiles - tiles % sms);
+            args2.tail_split = parts;
+            args2.tail_rec = sc.partials;
+            units = args2.full_tiles + (tiles % sms) * parts;
+        } else if (parts > 1) {
+            cudaGetLastError();  // no memory for the records: every tile is computed whole
+        }
+    }
+    const int grid = (int)(units < sms ? units : sms);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(KIND == 3 ? NTHREADS : 64 + 32 * EPI_WARPS_16);
@@ -1181,40 +1251,13 @@ int launch_cfg(const void *a0, const void *a1, const void *b, size_t lda, size_t
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
     XN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, ma0, ma1, mb, args2));
-    return XN_OK;
-}
-
-// Split-k for a product with too few 128 x 256 tiles to occupy the machine (a hundred-odd rows against a narrow
-// weight): `chunks` equal k ranges ride the tiled kernel's batch dimension (the operands' batch stride is the chunk
-// length along k), every (chunk, tile) leaves as an f32 record in library scratch, and splitk_reduce_kernel adds the
-// chunks in k order and applies the epilogue.  Narrow tiles would fill the SMs too, but every one of them re-reads the
-// whole A tile: 256 x 4096 x 4096 as 128 tiles of 128 x 64 pulls 196 MB through L2 for 36 MB of operands.
-template <int KIND, int NA>
-int launch_split_k(const void *a0, const void *a1, const void *b, size_t lda, size_t ldb, const GemmArgs &args, int chunks,
-                   cudaStream_t st) {
-    constexpr int bn = 256;
-    const long long num_m = (args.M + BM - 1) / BM, num_n = (args.N + bn - 1) / bn;
-    void *scratch = nullptr;
-    if (int rc = library_scratch(st, (size_t)chunks * num_m * num_n * bn * BM * sizeof(float), &scratch)) return rc;
-    GemmArgs a2 = args;
-    a2.K = args.K / chunks;
-    a2.batch = chunks;
-    a2.split_out = static_cast<float *>(scratch);
-    a2.col_bias = nullptr;
-    BatchGeom bg;
-    bg.batch = (size_t)chunks; bg.a_stride = (size_t)a2.K; bg.b_stride = (size_t)a2.K;
-    if (int rc = launch_cfg<KIND, bn, NA>(a0, a1, b, lda, ldb, a2, st, bg)) return rc;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(num_m * num_n * (bn / 8)));
-    cfg.blockDim = dim3(256);
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    XN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, splitk_reduce_kernel<KIND>, args.y[0], args.ldy, (const float *)scratch, chunks, args.M,
-                                     args.N, bn, args.x_scale, args.w_scale, args.col_bias));
+    if constexpr (KIND != 3) {
+        if (args2.tail_split > 1) {
+            const int num_m = (args.M + bmt_rows - 1) / bmt_rows, num_n = (args.N + BN - 1) / BN;
+            return launch_dependent(tail_reduce_kernel<KIND>, dim3((unsigned)(tail * (BN / 8))), dim3(256), 0, st, args2, BN, nacc,
+                                    num_m * num_n, num_m, num_n);
+        }
+    }
     return XN_OK;
 }
 
@@ -1228,29 +1271,14 @@ int launch_kind(const void *a0, const void *a1, const void *b, size_t lda, size_
     const int sms = sm_count();
     static const int force_bn = [] { const char *e = getenv("XN_GEMM_BN"); return e ? atoi(e) : 0; }();
     const long long m_tiles = (long long)((args.M + BM - 1) / BM) * args.batch;
-    if constexpr (KIND != 3) {
-        // split-k when 128 x 256 tiles would leave three quarters of the SMs idle and every chunk keeps >= 16 k stages
-        // (measured: two chunks gain nothing -- 512 x 4096 x 4096 bf16 25.2 us either way -- and chunks of 8 stages lose:
-        // fp8 W8A8 256 x 4096 x 4096 13.6 -> 15.0 us)
-        static const int force_split = [] { const char *e = getenv("XN_GEMM_SPLITK"); return e ? atoi(e) : -1; }();
-        constexpr int BKE = BKB / (KIND == 0 ? 1 : 2);
-        const long long t256 = m_tiles * ((args.N + 255) / 256);
-        if (force_split != 0 && args.batch == 1 && !args.causal && !args.a_bcast && args.ndst == 1 && !args.mc && !args.b_mn &&
-            !args.row_bias && !args.rows2 && args.col_offset == 0 && t256 * 4 <= sms && args.N >= 256) {
-            int chunks = 0;
-            for (int c = 8; c >= 4; c >>= 1)
-                if (c * t256 <= sms && args.K % (c * BKE) == 0 && args.K / (c * BKE) >= 16) { chunks = c; break; }
-            if (force_split > 1 && args.K % (force_split * BKE) == 0) chunks = force_split;
-            if (chunks >= 2) return launch_split_k<KIND, NA>(a0, a1, b, lda, ldb, args, chunks, st);
-        }
-    }
     int best = 256;
-    long long best_cost = -1;
+    double best_cost = -1;
+    const bool may_cut = KIND != 3 && may_cut_tail(args, st);
+    const int num_kb = (args.K + BKB / (KIND == 0 ? 1 : 2) - 1) / (BKB / (KIND == 0 ? 1 : 2));
     const int bn_step = args.b_mn ? 64 : 32;  // an n-contiguous B arrives in 64-column blocks
     for (int bn = 256; bn >= 64; bn -= bn_step) {
         const long long tiles = m_tiles * ((args.N + bn - 1) / bn);
-        const long long waves = (tiles + sms - 1) / sms;
-        const long long cost = waves * (NA * BM + bn);
+        const double cost = tile_rounds(tiles, num_kb, NA, may_cut) * (NA * BM + bn);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = bn; }
     }
     if (force_bn >= 64 && force_bn <= 256 && force_bn % bn_step == 0) best = force_bn;
@@ -1266,7 +1294,8 @@ int launch_kind(const void *a0, const void *a1, const void *b, size_t lda, size_
         if (best == 256 && !args.causal && !args.a_bcast && args.ndst == 1 && !args.mc) {
             const long long n_tiles = (args.N + 255) / 256;
             const long long t1 = m_tiles * n_tiles, t2 = (long long)((args.M + 2 * BM - 1) / (2 * BM)) * args.batch * n_tiles;
-            const double c1 = (double)((t1 + sms - 1) / sms) * 1.0, c2 = (double)((t2 + sms - 1) / sms) * 1.84;
+            const double c1 = tile_rounds(t1, num_kb, 1, may_cut),
+                         c2 = tile_rounds(t2, num_kb, 2, may_cut) * 1.84;
             bool rows2 = t2 >= sms && args.K >= 1024 && c2 < 0.97 * c1;
             if (force_rows2 >= 0) rows2 = force_rows2 != 0;
             if (rows2) {
@@ -1282,7 +1311,7 @@ int launch_kind(const void *a0, const void *a1, const void *b, size_t lda, size_
         best_cost = -1;
         for (int bn = 128; bn >= 64; bn -= 32) {
             const long long tiles = m_tiles * ((args.N + bn - 1) / bn);
-            const long long cost = ((tiles + sms - 1) / sms) * (NA * BM + bn);
+            const double cost = (double)(((tiles + sms - 1) / sms) * (NA * BM + bn));
             if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = bn; }
         }
         switch (best) {

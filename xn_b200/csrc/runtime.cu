@@ -36,6 +36,7 @@ volatile unsigned *g_status[MAX_DEV];  // host-mapped status words (one page-loc
 struct StreamScratch {
     int dev;
     cudaStream_t st;
+    int slot;  // SCRATCH_MAIN or SCRATCH_TAIL: two users that may be part of one call
     SkinnyScratch s;
 };
 std::vector<StreamScratch> g_table;
@@ -109,7 +110,7 @@ int wait_ctx(WaitCtx *out) {
 // A stream that is being captured cannot allocate: it borrows the largest buffer of its device -- the one of the
 // stream that ran the same shapes before the capture, which is how a CUDA graph is normally warmed up -- and is
 // refused with a clear message when no buffer is large enough.
-int skinny_scratch(cudaStream_t st, size_t partial_bytes, size_t ncounters, SkinnyScratch *out) {
+int skinny_scratch(cudaStream_t st, size_t partial_bytes, size_t ncounters, SkinnyScratch *out, int slot) {
     int dev = 0;
     if (int rc = current_device(&dev)) return rc;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -118,12 +119,12 @@ int skinny_scratch(cudaStream_t st, size_t partial_bytes, size_t ncounters, Skin
     std::lock_guard<std::mutex> lock(g_mu);
     StreamScratch *e = nullptr;
     for (auto &t : g_table)
-        if (t.dev == dev && t.st == st) { e = &t; break; }
+        if (t.dev == dev && t.st == st && t.slot == slot) { e = &t; break; }
     if (capturing) {
         if (!e || e->s.partial_bytes < partial_bytes || e->s.ncounters < ncounters) {
             e = nullptr;
             for (auto &t : g_table)
-                if (t.dev == dev && t.s.partial_bytes >= partial_bytes && t.s.ncounters >= ncounters &&
+                if (t.dev == dev && t.slot == slot && t.s.partial_bytes >= partial_bytes && t.s.ncounters >= ncounters &&
                     (!e || t.s.partial_bytes > e->s.partial_bytes))
                     e = &t;
         }
@@ -135,7 +136,7 @@ int skinny_scratch(cudaStream_t st, size_t partial_bytes, size_t ncounters, Skin
         return XN_OK;
     }
     if (!e) {
-        g_table.push_back(StreamScratch{dev, st, SkinnyScratch()});
+        g_table.push_back(StreamScratch{dev, st, slot, SkinnyScratch()});
         e = &g_table.back();
     }
     SkinnyScratch &s = e->s;
