@@ -431,30 +431,38 @@ conv_pack_taps_tr_kernel(T *__restrict__ wp, const T *__restrict__ w, int cin, i
     }
 }
 
-// The same two repackings through shared memory, one block per (out channel, 64 input channels): the taps are
-// read in runs of kernel_size contiguous elements and written in runs of 64 contiguous channels, so every
+// The same two repackings through shared memory, one block per (out channel, cc = 64 or 256 input channels): the
+// taps are read in runs of kernel_size contiguous elements and written in runs of cc contiguous channels, so every
 // sector moves once (the per-element kernels above touch a sector per element on one side and are kept for
 // kernel sizes whose tile does not fit).  TR = false: source (ci, kk) at w[(co * cin + ci) * ksize + kk],
 // destination rows co * ksize + kk.  TR = true: source at w[(ci * cout + co) * ksize + kk], destination rows
 // ((r * cout + co) * taps + j) holding tap kk = r + stride * (taps - 1 - j) or zeros.
-constexpr int PK_CC = 64;
 template <typename T, bool TR>
-__device__ __forceinline__ void pack_taps_block(T *wp, const T *w, T *tile, int cin, int cout, int ksize, int stride, int taps, int co, int c0) {
-    const int pitch = ksize + 1;  // tile: [PK_CC][pitch]
+__device__ __forceinline__ void pack_taps_block(T *wp, const T *w, T *tile, int cin, int cout, int ksize, int stride, int taps, int co, int c0,
+                                                int cc) {
+    const int pitch = ksize + 1, total = cc * ksize;  // tile: [cc][pitch]
     const size_t ci_stride = TR ? (size_t)cout * ksize : (size_t)ksize;
     const T *base = TR ? w + (size_t)co * ksize : w + (size_t)co * cin * ksize;
-#pragma unroll 4
-    for (int e = threadIdx.x; e < PK_CC * ksize; e += 256) {
-        const int ci = (int)((unsigned)e / (unsigned)ksize), kk = e - ci * ksize;
-        T v = from_f32<T>(0.f);
-        if (c0 + ci < cin) v = ld_act(base + (size_t)(c0 + ci) * ci_stride + kk);
-        tile[ci * pitch + kk] = v;
+    constexpr int U = 8;  // loads in flight per thread
+    for (int e0 = threadIdx.x; e0 < total; e0 += 256 * U) {
+        T v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int e = e0 + 256 * u, ci = (int)((unsigned)e / (unsigned)ksize), kk = e - ci * ksize;
+            v[u] = from_f32<T>(0.f);
+            if (e < total && c0 + ci < cin) v[u] = ld_act(base + (size_t)(c0 + ci) * ci_stride + kk);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int e = e0 + 256 * u, ci = (int)((unsigned)e / (unsigned)ksize);
+            if (e < total) tile[e + ci] = v[u];  // ci * pitch + kk
+        }
     }
     __syncthreads();
     const int nslots = TR ? stride * taps : ksize;
-    const int ci = threadIdx.x & (PK_CC - 1);
+    const int ci = threadIdx.x & (cc - 1);
     if (c0 + ci >= cin) return;
-    for (int sl = threadIdx.x / PK_CC; sl < nslots; sl += 256 / PK_CC) {
+    for (int sl = threadIdx.x / cc; sl < nslots; sl += 256 / cc) {
         size_t row;
         int kk;
         if (TR) {
@@ -475,14 +483,14 @@ __device__ __forceinline__ void pack_taps_block(T *wp, const T *w, T *tile, int 
 template <typename T, bool TR>
 __global__ void __launch_bounds__(256)
 conv_pack_kernel(T *xt, T *wp, const T *x, const T *w, int cin, int cout, int length, int lead, int rows, int ksize, int stride, int taps,
-                 unsigned tap_blocks, unsigned tap_chunks, unsigned row_blocks, unsigned channel_blocks) {
+                 unsigned tap_blocks, unsigned tap_chunks, int cc, unsigned row_blocks, unsigned channel_blocks) {
     extern __shared__ __align__(16) unsigned char pk_smem[];
     T *tile = reinterpret_cast<T *>(pk_smem);
     dependent_begin();
     unsigned i = blockIdx.x;
     if (i < tap_blocks) {
-        const unsigned co = i / tap_chunks, cc = i - co * tap_chunks;
-        pack_taps_block<T, TR>(wp, w, tile, cin, cout, ksize, stride, taps, (int)co, (int)cc * PK_CC);
+        const unsigned co = i / tap_chunks, chunk = i - co * tap_chunks;
+        pack_taps_block<T, TR>(wp, w, tile, cin, cout, ksize, stride, taps, (int)co, (int)chunk * cc, cc);
     } else {
         i -= tap_blocks;
         const unsigned rb = i % row_blocks, t = i / row_blocks, cb = t % channel_blocks, b = t / channel_blocks;
@@ -544,21 +552,22 @@ conv_interleave_kernel(T *__restrict__ out, const T *__restrict__ d, const T *__
     }
 }
 
-// out[row][col] = sum over splits of part[s][row][col] (+ bias[row]), summed in split order; four loads in flight per thread
+// out[row][col] = sum over splits of part[s][row][col] (+ bias[row]), summed in split order; 16 loads in flight per thread (a
+// streaming step has 28 splits of an output that fills less than one round of blocks: a chain of latencies)
 __global__ void __launch_bounds__(256)
 conv_sum_partials_kernel(float *out, const float *part, const float *bias, int splits, size_t n, size_t total) {
     dependent_begin<false>();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
         float s = 0.f;
-        for (int k = 0; k < splits; k += 4) {
-            float v[4];
+        const float b = bias ? ld_act_f32(bias + i / n) : 0.f;
+        for (int k = 0; k < splits; k += 16) {
+            float v[16];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = k + j < splits ? ld_act_f32(part + (size_t)(k + j) * total + i) : 0.f;
+            for (int j = 0; j < 16; ++j) v[j] = k + j < splits ? ld_act_f32(part + (size_t)(k + j) * total + i) : 0.f;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) s += v[j];
+            for (int j = 0; j < 16; ++j) s += v[j];
         }
-        if (bias) s += ld_act_f32(bias + i / n);
-        out[i] = s;
+        out[i] = bias ? s + b : s;
     }
 }
 
@@ -628,17 +637,21 @@ int launch_conv_gemm(xn_dtype dt, T *dst, const T *src, const T *kernel, const T
     T *d = reinterpret_cast<T *>(ws + p.xt_bytes + p.wp_bytes);
     const int lead = TR ? p.taps - 1 : a.padding;
     const size_t wtotal = TR ? (size_t)a.stride * cout * p.taps * cin : (size_t)cout * a.ksize * cin;
-    const size_t pk_smem = (size_t)PK_CC * (a.ksize + 1) * sizeof(T), in_smem = (size_t)PI_C * 33 * sizeof(T);
+    // Input channels per block of taps: 256 (seven loads per thread at seven taps, a KB per output run) once that still makes
+    // two blocks per SM, else 64.  f32 512 x 512 x 7 taps as 4096 blocks of 64 channels: 8 us for the launch, mostly latency.
+    const size_t row_bytes = (size_t)(a.ksize + 1) * sizeof(T);
+    const int cc = cin >= 256 && (size_t)cout * ((cin + 255) / 256) >= (size_t)sm_count() * 2 && 256 * row_bytes <= 40 * 1024 ? 256 : 64;
+    const size_t pk_smem = cc * row_bytes, in_smem = (size_t)PI_C * 33 * sizeof(T);
     // blocks that repack the taps (none when their tile does not fit: then the per-element kernels do it) and the input
     const bool tiled_taps = pk_smem <= 40 * 1024;
-    const size_t tap_chunks = (size_t)(cin + PK_CC - 1) / PK_CC, tap_blocks = tiled_taps ? (size_t)cout * tap_chunks : 0;
+    const size_t tap_chunks = (size_t)(cin + cc - 1) / cc, tap_blocks = tiled_taps ? (size_t)cout * tap_chunks : 0;
     const size_t row_blocks = (size_t)(p.rows + 31) / 32, channel_blocks = (size_t)(cin + PI_C - 1) / PI_C;
     const size_t blocks_all = tap_blocks + row_blocks * channel_blocks * (size_t)a.batch;
     XN_REQUIRE(blocks_all <= 0x7fffffff, "conv: too many blocks in the repacking launch");
     const size_t smem = tiled_taps && pk_smem > in_smem ? pk_smem : in_smem;
     XN_ENSURE_SMEM((conv_pack_kernel<T, TR>), smem);
     if (int rc = launch_dependent(conv_pack_kernel<T, TR>, dim3((unsigned)blocks_all), dim3(256), smem, st, xt, wp, src, kernel, cin, cout,
-                                  a.length, lead, p.rows, a.ksize, a.stride, p.taps, (unsigned)tap_blocks, (unsigned)tap_chunks,
+                                  a.length, lead, p.rows, a.ksize, a.stride, p.taps, (unsigned)tap_blocks, (unsigned)tap_chunks, cc,
                                   (unsigned)row_blocks, (unsigned)channel_blocks))
         return rc;
     if (!tiled_taps) {
