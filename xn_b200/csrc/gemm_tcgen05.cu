@@ -1122,6 +1122,11 @@ tail_reduce_kernel(const GemmArgs args, int bn, int nacc, int tiles_per_batch, i
         const float xs = ld_act_f32(x_scale + row);
 #pragma unroll
         for (int e = 0; e < 4; ++e) val[e] = (col + e < N ? __ldg(w_scale + col + e) : 0.0f) * (xs * val[e]);
+    } else if (args.row_bias) {  // a convolution's output channel
+        const float rb = KIND == 2 ? __half2float(reinterpret_cast<const __half *>(args.row_bias)[row])
+                                   : __bfloat162float(reinterpret_cast<const __nv_bfloat16 *>(args.row_bias)[row]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) val[e] += rb;
     }
     uint16_t out[4];
 #pragma unroll
@@ -1152,14 +1157,16 @@ struct BatchGeom { size_t batch = 1, a_stride = 0, b_stride = 0; };
 // range written and read back through L2 and a launch that adds them: about 13 us at 128 x 256 tiles, tail_stages() k
 // stages.  us, no cut / cut: f16 3001 x 4096 x 11264 (192 tiles of 256 x 256: 148 + 44, three ranges) 230 / 202.5; bf16
 // 300 x 4096 x 8192 34.7 / 32.3; fp8 W8A16 4096 x 4096 x 11264 300 / 288.  Where the line is too low: bf16 1024 x 5120 x 4096
-// (64 stages) 39.5 / 42.6 at 24, 512 x 4096 x 4096 20.2 / 27.4 at 8; more than four ranges add records, not speed.
+// (64 stages) 39.5 / 42.6 at 24, 512 x 4096 x 4096 20.2 / 27.4 at 8; more than four ranges add records, not speed,
+// but where a handful of tiles is all there is.
 constexpr int TAIL_MAX_PARTS = 4;
 constexpr int TAIL_MIN_STAGES = 8;  // k stages per range
 constexpr int tail_stages(int na) { return na == 2 ? 16 : 32; }  // a stage of two A tiles takes about twice as long
 inline int tail_parts(long long tiles, int num_kb, int na) {
     const long long sms = sm_count(), tail = tiles % sms;
     if (tail == 0 || tail * 2 > sms) return 1;
-    long long parts = sms / tail < TAIL_MAX_PARTS ? sms / tail : TAIL_MAX_PARTS;
+    const long long most = tiles * 8 <= sms ? 8 : TAIL_MAX_PARTS;  // a product of a handful of tiles leaves the chip empty
+    long long parts = sms / tail < most ? sms / tail : most;
     if (parts > num_kb / TAIL_MIN_STAGES) parts = num_kb / TAIL_MIN_STAGES;
     return parts > 1 && num_kb - num_kb / parts > tail_stages(na) ? (int)parts : 1;
 }
@@ -1169,10 +1176,10 @@ inline double tile_rounds(long long tiles, int num_kb, int na, bool may_cut) {
     if (parts <= 1) return (double)((tiles + sms - 1) / sms);
     return (double)(tiles / sms) + 1.0 / (double)parts + (double)tail_stages(na) / num_kb;
 }
-// A captured launch may be replayed beside anything: it takes no scratch it would share.  Peers' buffers and the
-// convolutions' row bias stay with the tiled kernel's own epilogue.
+// A captured launch may be replayed beside anything: it takes no scratch it would share.  Peers' buffers stay with
+// the tiled kernel's own epilogue.
 inline bool may_cut_tail(const GemmArgs &a, cudaStream_t st) {
-    if (a.causal || a.ndst != 1 || a.mc || a.row_bias) return false;
+    if (a.causal || a.ndst != 1 || a.mc) return false;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
 }
