@@ -15,18 +15,17 @@
  * host threads at once (the reference's Backend is Send + Sync,
  * xn-core/src/backend.rs:4).
  *
- * Library-owned device memory: one kernel (the skinny tensor-memory form, used by xn_mm_gemm for
- * 16-bit operands with 17..64 rows, or fewer rows and a very long k, and by the fp8 linears for 9..64
- * rows) hands split tiles over through a buffer per (device, stream) that the library allocates when a
- * stream first needs it and grows when a larger problem arrives (a few MB; cudaMalloc, i.e. not allowed
- * during stream capture: run each shape once before capturing it, as a decode loop does anyway; a stream
- * under capture borrows the buffer of the stream that ran those shapes, so keep the graph's replays ordered
- * with that stream's own calls).  Calls on different streams use different buffers and may overlap.
- * The same buffer holds the repacked operands of an f32 xn_mm_gemm with 17 or more rows (three tf32
- * pieces per element: 12 bytes per operand element, refused above 2 GiB in favour of the plain f32
- * kernel; XN_MM_F32_TC=0 in the environment keeps every f32 call on the plain kernel).
+ * Library-owned device memory: buffers per (device, stream) that the library allocates when a stream first needs
+ * them and grows when a larger problem arrives (cudaMalloc, i.e. not allowed during stream capture: run each shape
+ * once before capturing it, as a decode loop does anyway; a stream under capture borrows the buffer of the stream
+ * that ran those shapes, so keep the graph's replays ordered with that stream's own calls).  Calls on different
+ * streams use different buffers and may overlap.  They hold the repacked operands of an f32 xn_mm_gemm with 17 or
+ * more rows (three tf32 pieces per element: 12 bytes per operand element, refused above 2 GiB in favour of the plain
+ * f32 kernel; XN_MM_F32_TC=0 in the environment keeps every f32 call on the plain kernel), unpacked block weights,
+ * lhs rows copied to a pitch TMA can address, and the partial sums of output tiles that the tiled tensor-memory
+ * kernel cuts along k (up to 76 MB; a captured launch, or one for which there is no memory, cuts none).
  * Nothing else allocates;
- * xn_mm_linear_fp8_noalloc avoids that kernel altogether.
+ * xn_mm_linear_fp8_noalloc runs only kernels that need none of it.
  */
 #ifndef XN_MM_H
 #define XN_MM_H
@@ -73,8 +72,8 @@ int xn_mm_abi_version(void);
  * Library-owned scratch (see the top of this file) is kept per (device, stream) for the life of the process;
  * a replaced block is kept too, since a captured graph may still point at it.  xn_mm_release_scratch
  * synchronises the current device and frees the blocks of `stream` (or of every stream when all_streams != 0)
- * together with all replaced blocks of the device; graphs captured earlier that ran the skinny kernel or the
- * f32 repack must not be replayed afterwards.
+ * together with all replaced blocks of the device; graphs captured earlier that ran a call which
+ * uses them must not be replayed afterwards.
  * ------------------------------------------------------------------------------------------ */
 int xn_mm_device_status(unsigned *timeouts_out);
 int xn_mm_clear_device_status(void);
