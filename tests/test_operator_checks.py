@@ -1,0 +1,24 @@
+"""What the operators refuse before anything is allocated or launched.  The checks need no device, so they run on CPU tensors."""
+import pytest
+import torch
+
+
+@pytest.mark.parametrize("shape", [(4, 512), (4, 128), (1, 512), (2, 2, 512), (2, 3, 128), (4, 257), (512,), (128,), (4, 0), ()])
+def test_int4_layer_refuses_rows_of_another_width(xn, shape):
+    """Rows of 2 k elements would be twice as many rows as the output has, rows of k / 2 half as many."""
+    layer = xn.LinearQ4(torch.zeros(16 * 256, dtype=torch.uint8), 16, 256)
+    with pytest.raises(xn.XnError, match="rows of 256 elements"):
+        layer(torch.zeros(shape))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(3, 256), (256,), (2, 3, 256), (0, 256), (2, 0, 256), (0, 7)])
+def test_int4_layer_takes_any_leading_dimensions(xn, cuda, shape):
+    g = torch.Generator(device=cuda).manual_seed(1)
+    layer = xn.LinearQ4.from_weight(torch.randn(48, 256, generator=g, device=cuda))
+    x = torch.randn(*shape, generator=g, device=cuda)
+    y = layer(x)
+    assert y.shape == (*shape[:-1], 48)
+    if x.numel():
+        xq, xs = xn.quantize_rows_i8(x.reshape(-1, 256))
+        assert torch.equal(y.reshape(-1, 48), xn.linear_q4(xq, xs, layer.wq, 48))

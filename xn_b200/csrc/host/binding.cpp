@@ -219,11 +219,15 @@ XN_BINDING(linear, 3) {
 // ---------------------------------------------------------------------------------------------
 // Quantized linears
 // ---------------------------------------------------------------------------------------------
-// x as contiguous rows of k elements; `keep` holds the copy a non-contiguous view needs
-const at::Tensor &rows_of(const at::Tensor &x, int64_t k, at::Tensor &keep) {
-    if (x.is_contiguous() && x.dim() >= 1 && x.size(-1) == k) return x;
-    keep = x.reshape({-1, k}).contiguous();
-    return keep;
+// The rows of x [..., k], counted over its leading dimensions, which are also the output's: a last dimension that is not the
+// layer's k is refused here, before anything is allocated or launched (as many rows of k elements as x holds would not be as
+// many as the output has).
+size_t rows_in(const char *name, const at::Tensor &x, int64_t k) {
+    size_t m = 1;
+    for (int64_t i = 0; i + 1 < x.dim(); ++i) m *= (size_t)x.size(i);
+    if (x.dim() < 1 || (m != 0 && x.size(-1) != k))
+        raise_xn(XN_ERR_INVALID, "%s expects rows of %lld elements, got %s", name, (long long)k, shape_text(x).c_str());
+    return m;
 }
 
 XN_BINDING(quantize_rows_i8, 3) {  // x [m, k], xq or None, x_scale or None
@@ -282,11 +286,10 @@ XN_BINDING(linear_block, 7) {  // bits, xq, x_scale, packed weights, n, partials
 XN_BINDING(linear_q4_forward, 4) {  // x [..., k], packed weights, n, k: quantize the rows, then the linear
     const at::Tensor &x = tensor(a[0]), &wq = tensor(a[1]);
     const int64_t n = (int64_t)size_arg(a[2]), k = (int64_t)size_arg(a[3]);
+    const size_t m = rows_in("linear_q4", x, k);
     require_cuda(x);
     require_cuda(wq);
-    at::Tensor keep;
-    const at::Tensor &xr = rows_of(x, k, keep);
-    const size_t m = k ? (size_t)(xr.numel() / k) : 0;
+    const at::Tensor xr = x.contiguous();
     const xn_dtype dt = dtype_code(x.scalar_type());
     // codes and row scales in one block, the scales behind the codes at a 256-byte boundary
     const size_t codes = (m * (size_t)k + 255) / 256 * 256;
@@ -337,8 +340,7 @@ XN_BINDING(linear_fp8, 6) {  // x [..., k] bf16, weights, scales, variant, works
     require_cuda(wq);
     if (x.scalar_type() != at::kBFloat16) raise_xn(XN_ERR_INVALID, "linear_fp8 takes bf16 activations");
     const int64_t k = x.size(-1), n = wq.size(0);
-    at::Tensor keep;
-    const at::Tensor &xr = rows_of(x, k, keep);
+    const at::Tensor xr = x.contiguous();
     const size_t m = k ? (size_t)(xr.numel() / k) : 0;
     const size_t need = xn_mm_linear_fp8_workspace_bytes(m, (size_t)k);
     at::Tensor ws = work ? *work : empty({(int64_t)need}, at::kByte, x.device());
