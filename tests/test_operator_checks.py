@@ -11,6 +11,30 @@ def test_int4_layer_refuses_rows_of_another_width(xn, shape):
         layer(torch.zeros(shape))
 
 
+@pytest.mark.parametrize("shape", [(4, 512), (4, 128), (2, 2, 272), (128,), ()])
+def test_fp8_layer_refuses_rows_of_another_width(xn, shape):
+    """Longer rows would read past the weight's end."""
+    layer = xn.LinearFp8(torch.zeros(16, 256, dtype=torch.uint8), torch.ones(16))
+    with pytest.raises(xn.XnError, match="rows of 256 elements"):
+        layer(torch.zeros(shape, dtype=torch.bfloat16))
+
+
+def test_fp8_linear_takes_a_matrix(xn):
+    with pytest.raises(xn.XnError, match="a matrix"):
+        xn.linear_fp8(torch.zeros(2, 3, 256, dtype=torch.bfloat16), torch.zeros(16, 256, dtype=torch.uint8), torch.ones(16))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(3, 256), (256,), (2, 3, 256), (0, 256)])
+def test_fp8_layer_takes_any_leading_dimensions(xn, cuda, shape):
+    g = torch.Generator(device=cuda).manual_seed(1)
+    layer = xn.LinearFp8.from_weight(torch.randn(48, 256, generator=g, device=cuda))
+    x = torch.randn(*shape, generator=g, device=cuda).bfloat16()
+    y = layer(x)
+    assert y.shape == (*shape[:-1], 48)
+    assert torch.equal(y.reshape(-1, 48), xn.linear_fp8(x.reshape(-1, 256), layer.wq, layer.ws))
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("shape", [(3, 256), (256,), (2, 3, 256), (0, 256), (2, 0, 256), (0, 7)])
 def test_int4_layer_takes_any_leading_dimensions(xn, cuda, shape):

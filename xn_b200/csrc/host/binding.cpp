@@ -336,12 +336,12 @@ XN_BINDING(linear_fp8, 6) {  // x [..., k] bf16, weights, scales, variant, works
     const at::Tensor &x = tensor(a[0]), &wq = tensor(a[1]), &wsc = tensor(a[2]);
     const int variant = (int)size_arg(a[3]);
     const at::Tensor *work = maybe_tensor(a[4]), *out = maybe_tensor(a[5]);
+    const int64_t n = wq.size(0), k = n ? wq.numel() / n : x.size(-1);  // a weight holds whole rows of k bytes
+    const size_t m = rows_in("linear_fp8", x, k);
     require_cuda(x);
     require_cuda(wq);
     if (x.scalar_type() != at::kBFloat16) raise_xn(XN_ERR_INVALID, "linear_fp8 takes bf16 activations");
-    const int64_t k = x.size(-1), n = wq.size(0);
     const at::Tensor xr = x.contiguous();
-    const size_t m = k ? (size_t)(xr.numel() / k) : 0;
     const size_t need = xn_mm_linear_fp8_workspace_bytes(m, (size_t)k);
     at::Tensor ws = work ? *work : empty({(int64_t)need}, at::kByte, x.device());
     at::Tensor y;

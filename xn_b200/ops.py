@@ -233,6 +233,8 @@ def split_rows_e4m3(x: torch.Tensor, want_lo: bool = True):
 def linear_fp8(x: torch.Tensor, wq: torch.Tensor, w_scale: torch.Tensor, variant: int = 0,
                workspace: torch.Tensor | None = None, out: torch.Tensor | None = None) -> torch.Tensor:
     """y bf16 [m,n] = fp8 linear of bf16 x [m,k]; variant 0 = W8A16, 1 = W8A8."""
+    if x.dim() != 2:
+        raise XnError(_lib.ERR_INVALID, f"linear_fp8 expects a matrix of activations, got {list(x.shape)}")
     return _host.linear_fp8(x, wq, w_scale, variant, workspace, out)
 
 
