@@ -232,10 +232,13 @@ rms_norm_vec_kernel(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T *src
     const float denom = sqrtf(s2 / (float)cols + eps), rden = __frcp_rn(denom);
     // x / denom for every element from the row's one reciprocal: with rden = RN(1 / denom), q = x * rden and the residual
     // x - q * denom (exact in an fma), q + residual * rden is the correctly rounded quotient (Markstein's theorem on
-    // division by a correctly rounded reciprocal; outside the subnormal range).
+    // division by a correctly rounded reciprocal; outside the subnormal range).  A row whose sum of squares overflows has
+    // denom = inf and one of zeros without an epsilon denom = 0: there x * rden is x / denom for every x (0, inf and NaN
+    // included), and the residual would be NaN.
+    const bool regular = rden > 0.0f && rden < INFINITY;
     auto quotient = [&](float x) {
-        const float q = x * rden;
-        return fmaf(fmaf(-q, denom, x), rden, q);
+        const float q = x * rden, r = fmaf(-q, denom, x);
+        return regular ? fmaf(r, rden, q) : q;
     };
     float amax = 0.0f;
 #pragma unroll
