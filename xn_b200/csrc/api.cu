@@ -100,6 +100,11 @@ static int gemm_dispatch(xn_dtype dtype, void *dst, const void *lhs, size_t lhs_
                "gemm: unsupported dst strides (%zu, %zu) for m:%zu n:%zu", dst_cs, dst_rs, m, n);
     const char *l = static_cast<const char *>(lhs) + lhs_off * es;
     const char *r = static_cast<const char *>(rhs) + rhs_off * es;
+    // An empty reduction is zeros.  The kernel below, which reads no operand then, writes them at any strides; the others walk
+    // k in steps of theirs and are entered with one element at least.
+    if (k == 0 && !causal)
+        return launch_gemm_generic(dtype, dst, l, r, m, n, k, lhs_b, lhs_b_stride, rhs_b_stride, dst_cs, dst_rs, lhs_cs, lhs_rs,
+                                   rhs_cs, rhs_rs, (cudaStream_t)stream);
     // Decode-sized matmul_t with 16-bit elements (m <= 16, one batch, both operands k-contiguous, a weight worth
     // streaming): the tensor-core weight-streaming kernel.  (Its mma.sync instructions issue at about one per 32
     // cycles per SM sub-partition on this architecture -- 1/16 of the tcgen05 rate -- so beyond two column groups

@@ -149,6 +149,13 @@ template <typename F> PyObject *guarded(F &&body) {
 // ---------------------------------------------------------------------------------------------
 // matmul / Linear (xn-core/src/ops.rs:631-714, inplace_ops.rs:318-436, nn/linear.rs:4-71)
 // ---------------------------------------------------------------------------------------------
+// Where a view begins in its storage, also when it has no elements (data_ptr() is null then): a product over no elements
+// is zeros, and a live tensor's empty slice is a valid operand of it.
+const void *view_ptr(const at::Tensor &t) {
+    const char *base = static_cast<const char *>(t.storage().data());
+    return base ? base + (size_t)t.storage_offset() * t.itemsize() : nullptr;
+}
+
 void matmul_into(const at::Tensor &dst, const at::Tensor &lhs, const at::Tensor &rhs, bool rhs_t) {
     require_cuda(dst);
     require_cuda(lhs);
@@ -163,7 +170,7 @@ void matmul_into(const at::Tensor &dst, const at::Tensor &lhs, const at::Tensor 
     size_t p[12];
     check(xn_mm_matmul_plan((size_t)lhs.dim(), ls, lt, (size_t)rhs.dim(), rs, rt, rhs_t ? 1 : 0, (size_t)dst.numel(), p));
     void *d = dst.data_ptr();
-    const void *l = lhs.data_ptr(), *r = rhs.data_ptr();
+    const void *l = view_ptr(lhs), *r = view_ptr(rhs);
     void *st = stream();
     XN_CALL(xn_mm_gemm(dt, d, l, 0, r, 0, p[0], p[1], p[2], p[3], p[4], p[5], p[6], p[7], p[8], p[9], p[10], p[11], st));
 }
@@ -200,10 +207,10 @@ XN_BINDING(linear, 3) {
                      dtype_name(x.scalar_type()), shape_text(*b).c_str(), dtype_name(b->scalar_type()));
     }
     if (!(x.is_cuda() && w.is_cuda() && x.scalar_type() == w.scalar_type() && x.dim() >= 2 && w.dim() == 2 &&
-          x.size(-1) == w.size(1) && w.stride(1) == 1 && x.is_contiguous()))
+          x.size(-1) == w.size(1) && w.size(1) != 0 && w.stride(1) == 1 && x.is_contiguous()))
         Py_RETURN_NONE;
     const xn_dtype dt = dtype_code(x.scalar_type());
-    const size_t n = (size_t)w.size(0), k = (size_t)w.size(1), m = k ? (size_t)x.numel() / k : 0, ldw = (size_t)w.stride(0);
+    const size_t n = (size_t)w.size(0), k = (size_t)w.size(1), m = (size_t)x.numel() / k, ldw = (size_t)w.stride(0);
     Shape s;
     s.lead(x, x.dim() - 1);
     s.d.push_back((int64_t)n);
