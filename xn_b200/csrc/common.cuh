@@ -237,6 +237,18 @@ constexpr int SCRATCH_MAIN = 0;  // operands repacked for a launch, split sums
 constexpr int SCRATCH_TAIL = 1;  // the tiled kernel's records of cut tiles: its operands may lie in the other buffer
 int skinny_scratch(cudaStream_t st, size_t partial_bytes, size_t ncounters, SkinnyScratch *out, int slot = SCRATCH_MAIN);
 int library_scratch(cudaStream_t st, size_t bytes, void **out);
+// Held by a call that hands data from one of its launches to the next through library scratch, from the lookup to the last
+// launch: another host thread's call on the same stream must not enqueue between them and overwrite the scratch.  One lock
+// per (device, stream), so a thread whose launch blocks on a full queue holds up nobody else's stream; recursive, because
+// such a call may be part of another.
+struct ScratchHold {
+    explicit ScratchHold(cudaStream_t st);
+    ~ScratchHold();
+    ScratchHold(const ScratchHold &) = delete;
+    ScratchHold &operator=(const ScratchHold &) = delete;
+private:
+    void *mu;  // std::recursive_mutex, kept for the life of the process
+};
 struct WaitCtx;
 // Fills the bound and the status-word pointer every kernel with device-side waits takes; fails with
 // XN_ERR_DEVICE when an earlier launch on the current device has reported a wait that ran out.

@@ -89,6 +89,7 @@ int launch_gemm_f32_tc(float *dst, const float *lhs, const float *rhs, size_t m,
     const size_t xbytes = (m * k * 12 + 255) / 256 * 256, wbytes = (n * k * 12 + 255) / 256 * 256;
     const int splits = k_splits(m, n, 3 * k);
     const size_t pbytes = splits > 1 ? (size_t)splits * m * n * 4 : 0;
+    ScratchHold hold(st);
     if (int rc = library_scratch(st, xbytes + wbytes + pbytes, &ws)) return rc;
     float *xp = static_cast<float *>(ws), *wp = reinterpret_cast<float *>(static_cast<unsigned char *>(ws) + xbytes);
     // lhs element (i, p) at i * lhs_rs + p * lhs_cs; rhs element (p, j) at p * rhs_rs + j * rhs_cs: row j of the

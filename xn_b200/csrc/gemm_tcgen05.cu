@@ -28,6 +28,8 @@
 //
 // Every mbarrier wait is bounded in time (wait.cuh); a wait that gives up reports it through the device's
 // host-visible status word and the CTA drains through its common exit (tensor memory is always released).
+#include <optional>
+
 #include "tc05.cuh"
 
 namespace xn {
@@ -1234,9 +1236,11 @@ int launch_cfg(const void *a0, const void *a1, const void *b, size_t lda, size_t
     args2.tail_split = 1;
     const int nacc = NA == 2 && args.rows2 ? 2 : 1;
     const size_t tail = (size_t)(tiles % sms) * nacc;
+    std::optional<ScratchHold> hold;  // from the records' lookup to the launch that adds them
     if (KIND != 3 && may_cut_tail(args, st)) {
         const int parts = tail_parts(tiles, (args.K + BKB / ELEM - 1) / (BKB / ELEM), NA);
         SkinnyScratch sc;
+        if (parts > 1) hold.emplace(st);
         if (parts > 1 && skinny_scratch(st, tail * parts * BN * BM * sizeof(float), 0, &sc, SCRATCH_TAIL) == XN_OK) {
             args2.full_tiles = (int)(tiles - tiles % sms);
             args2.tail_split = parts;

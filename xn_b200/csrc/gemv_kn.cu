@@ -308,6 +308,7 @@ int launch_gemm_kn_repitched(xn_dtype dt, void *dst, const void *lhs, const void
                              size_t lhs_bs, size_t rhs_bs, size_t dst_rs, size_t lhs_rs, size_t rhs_rs, cudaStream_t st) {
     const size_t lda = (k + 7) / 8 * 8, rows = batch * m;
     void *tmp = nullptr;
+    ScratchHold hold(st);
     if (int rc = library_scratch(st, rows * lda * 2, &tmp)) return rc;
     const size_t blocks = (rows + 7) / 8, most = (size_t)sm_count() * 8;
     if (int rc = launch_dependent(repitch_rows_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, st,

@@ -591,6 +591,7 @@ int linear_q_tensor(float *y, const int8_t *xq, const float *x_scale, const void
     const size_t n_pad = (n + 15) / 16 * 16, nblk = k / 32;
     const size_t w_bytes = (n_pad * k + 255) / 256 * 256;
     void *ws = nullptr;
+    ScratchHold hold(st);
     if (int rc = library_scratch(st, w_bytes + n_pad * nblk * sizeof(float), &ws)) return rc;
     int8_t *w8 = static_cast<int8_t *>(ws);
     float *scales = reinterpret_cast<float *>(static_cast<unsigned char *>(ws) + w_bytes);

@@ -1457,6 +1457,7 @@ extern "C" int xn_mm_decode_attention_append_e4m3(uint8_t *x_hi, uint8_t *x_lo, 
     bool in_kernel = batch * heads * (size_t)splits <= (size_t)sm_count() * 5 * 2;
     if (merge) in_kernel = merge == 1;
     if (in_kernel) {
+        ScratchHold hold(st);
         SkinnyScratch sc;  // arrival counters: one per (stream, head), one per stream; zero between launches
         if (int rc = skinny_scratch(st, 0, batch * heads + batch, &sc)) return rc;
         decode_attention_append_kernel<true><<<dim3((unsigned)(batch * heads), (unsigned)splits), 128, 0, st>>>(

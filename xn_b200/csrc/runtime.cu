@@ -7,7 +7,10 @@
 // lives in pinned, mapped host memory: the host reads it without synchronising, every later launch on that
 // device is refused with XN_ERR_DEVICE until xn_mm_clear_device_status(), and xn_mm_device_status() lets a
 // caller poll it at its own synchronisation points.
+#include <map>
+#include <memory>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
@@ -45,6 +48,8 @@ std::vector<StreamScratch> g_table;
 // stays here until xn_mm_release_scratch().
 struct Retired { int dev; void *p; };
 std::vector<Retired> g_retired;
+// ScratchHold's locks.  Taken before g_mu, never while holding it; a thread holds at most one stream's.
+std::map<std::pair<int, cudaStream_t>, std::unique_ptr<std::recursive_mutex>> g_holds;
 
 thread_local bool tl_no_alloc = false;
 
@@ -72,6 +77,21 @@ __global__ void selftest_wait_kernel(WaitCtx w, unsigned *gave_up) {
 
 NoAllocScope::NoAllocScope() : prev(tl_no_alloc) { tl_no_alloc = true; }
 NoAllocScope::~NoAllocScope() { tl_no_alloc = prev; }
+
+ScratchHold::ScratchHold(cudaStream_t st) {
+    int dev = -1;
+    cudaGetDevice(&dev);  // a failure shows in the lookup that follows
+    std::recursive_mutex *m;
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        auto &slot = g_holds[{dev, st}];
+        if (!slot) slot = std::make_unique<std::recursive_mutex>();
+        m = slot.get();
+    }
+    m->lock();
+    mu = m;
+}
+ScratchHold::~ScratchHold() { static_cast<std::recursive_mutex *>(mu)->unlock(); }
 
 int wait_ctx(WaitCtx *out) {
     int dev = 0;
@@ -200,6 +220,17 @@ extern "C" int xn_mm_release_scratch(void *stream, int all_streams) {
     XN_API_RANGE("xn_mm_release_scratch");
     int dev = 0;
     if (int rc = current_device(&dev)) return rc;
+    // no call is between its scratch lookup and its last launch while blocks are freed
+    std::vector<std::unique_lock<std::recursive_mutex>> holds;
+    {
+        std::vector<std::recursive_mutex *> all;
+        {
+            std::lock_guard<std::mutex> lock(g_mu);
+            for (auto &h : g_holds)
+                if (h.first.first == dev) all.push_back(h.second.get());
+        }
+        for (auto *m : all) holds.emplace_back(*m);
+    }
     XN_CHECK_CUDA(cudaDeviceSynchronize());
     std::lock_guard<std::mutex> lock(g_mu);
     for (size_t i = 0; i < g_table.size();) {
