@@ -148,7 +148,8 @@ linear_q4_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const flo
     const int nblk = k / 32, nsb = k / 128;
     const int nwarps = blockDim.x >> 5;
     // [rings: nwarps * depth slots of UPC units, reused as red: nwarps * MT*4*32 f32]
-    // [activations: 8*MT rows of k int8 at a pitch of k+16 bytes][mbarriers: nwarps * depth, then one per k slice for the activations]
+    // [activations: 8*MT rows of k int8 at a pitch of k+16 bytes][mbarriers: nwarps * depth, then MAX_WARPS, one per k slice, for the activations]
+    // [x_scale of the rows: 16 f32]
     unsigned char *rings = smem;
     constexpr int slot_bytes = UPC * UNIT_BYTES;
     unsigned char *sX = smem + (size_t)nwarps * depth * slot_bytes;
@@ -205,14 +206,13 @@ linear_q4_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const flo
         for (int r = 0; r < rows; ++r)
             bulk_load(sX + (size_t)r * pitch + (size_t)sb0 * 128, xq + (size_t)r * k + (size_t)sb0 * 128, bytes, &xbars[ks]);
     }
-    float xs_reg[MT][2];  // x_scale of the activation rows this lane stores at the end
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int row_m = 8 * mt + 2 * t + e;
-            xs_reg[mt][e] = row_m < m ? ld_act_f32(x_scale + row_m) : 0.0f;
-        }
+    // x_scale of the at most 16 activation rows: one request per CTA, handed to the storing warps through shared memory behind
+    // the unit loops.  (The load is coherent -- the quantizer may have run beside this CTA's start -- and so served by L2: asked
+    // by every warp for itself, 6 to 12 thousand requests for one sector ahead of the ring fill, 16 x 11264 x 4096 took 11.2 us
+    // against 8.5.)
+    float *s_xs = reinterpret_cast<float *>(xbars + MAX_WARPS);
+    float xs_mine = 0.0f;
+    if (warp == 0 && lane < min(m, 8 * MT)) xs_mine = ld_act_f32(x_scale + lane);
     // The rest of the first ring-full.  With few activation rows it goes out at once.  From 6 rows on the
     // activation copies (24+ KB per SM, wanted before any MMA can start) would share the SM's copy
     // bandwidth with 100 KB of weights that are not needed yet: there the ring is filled only after the
@@ -286,8 +286,9 @@ linear_q4_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const flo
     }
 
     // Fixed-order reduction over the ksplit warps of a tile.
+    if (warp == 0 && lane < 8 * MT) s_xs[lane] = xs_mine;
+    __syncthreads();  // all unit loops are over: the ring area becomes the reduction buffer
     if (ksplit > 1) {
-        __syncthreads();  // all unit loops are over: the ring area becomes the reduction buffer
         if (ks > 0) {
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt)
@@ -311,7 +312,7 @@ linear_q4_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const flo
             for (int e = 0; e < 4; ++e) {
                 const size_t row_n = (size_t)tile * 16 + g + 8 * (e >> 1);
                 const int row_m = 8 * mt + 2 * t + (e & 1);
-                if (row_n < n && row_m < m) y[(size_t)row_m * n + row_n] = xs_reg[mt][e & 1] * (acc[mt][e] * (BITS == 4 ? 0.0625f : 1.0f));
+                if (row_n < n && row_m < m) y[(size_t)row_m * n + row_n] = s_xs[row_m] * (acc[mt][e] * (BITS == 4 ? 0.0625f : 1.0f));
             }
     }
 }
@@ -328,9 +329,15 @@ linear_q4_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const flo
 // ---------------------------------------------------------------------------------------------
 constexpr int TK_WARPS = 4;    // k split inside a CTA
 
+__device__ __forceinline__ unsigned ld_u32(const unsigned *p) {
+    unsigned v;
+    asm("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+
 template <int MT, bool DUMP, int BITS>
 __global__ void __launch_bounds__(TK_WARPS * 32, 5)
-linear_q_tile_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const float *__restrict__ x_scale,
+linear_q_tile_kernel(float *__restrict__ y, const int8_t *xq, const float *x_scale,
                      const unsigned char *__restrict__ wq, int m, size_t n, int k, int32_t *__restrict__ partials, const WaitCtx wctx) {
     constexpr int UNIT_BYTES = Tile<BITS>::UNIT;
     constexpr int SU = BITS == 4 ? 4 : 2;  // units per ring slot: 5 KB either way (static shared memory < 48 KB)
@@ -369,6 +376,10 @@ linear_q_tile_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const
 
     // Activation words of block kb for column group mt: {xq[8mt+g][32kb+4t..], xq[8mt+g][32kb+16+4t..]}.
     // Rows past m are clamped to row m-1: their columns of the product are computed and dropped.
+    // Ordinary loads: they see what the wait made visible, and L1 serves the other CTAs of the SM (through L2 alone 16 x 4096 x
+    // 11264 took 33.6 us, 17.2 with reuse).  The pointer is made anew behind the wait, so none is moved ahead of it; between
+    // themselves, the math and the waits for weights the compiler may move them (nothing here writes xq).
+    asm volatile("" : "+l"(xq));
     const int8_t *xrow[MT];
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) xrow[mt] = xq + (size_t)min(8 * mt + g, m - 1) * k + (size_t)sb0 * 128 + 4 * t;
@@ -389,8 +400,8 @@ linear_q_tile_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const
             const unsigned *src = reinterpret_cast<const unsigned *>(xrow[mt] + (size_t)i * 128);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                b[mt][2 * j] = __float_as_uint(ld_act_f32(reinterpret_cast<const float *>(src + 8 * j)));
-                b[mt][2 * j + 1] = __float_as_uint(ld_act_f32(reinterpret_cast<const float *>(src + 8 * j + 4)));
+                b[mt][2 * j] = ld_u32(src + 8 * j);
+                b[mt][2 * j + 1] = ld_u32(src + 8 * j + 4);
             }
         }
     };
@@ -434,11 +445,18 @@ linear_q_tile_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const
 #pragma unroll
             for (int e = 0; e < 4; ++e) acc[mt][e] = __int_as_float(0x7fc00000);
     }
+    float xs_reg[MT][2] = {};  // the storing warp's row scales, in flight together while the others hand over
     if (warp > 0) {
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
             for (int e = 0; e < 4; ++e) red[warp][mt * 4 + e][lane] = acc[mt][e];
+    } else {
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+                if (8 * mt + 2 * t + e < m) xs_reg[mt][e] = ld_act_f32(x_scale + 8 * mt + 2 * t + e);
     }
     __syncthreads();
     if (warp == 0) {
@@ -455,7 +473,7 @@ linear_q_tile_kernel(float *__restrict__ y, const int8_t *__restrict__ xq, const
                 const size_t row_n = (size_t)tile * 16 + g + 8 * (e >> 1);
                 const int row_m = 8 * mt + 2 * t + (e & 1);
                 if (row_n < n && row_m < m)
-                    y[(size_t)row_m * n + row_n] = ld_act_f32(x_scale + row_m) * (acc[mt][e] * (BITS == 4 ? 0.0625f : 1.0f));
+                    y[(size_t)row_m * n + row_n] = xs_reg[mt][e & 1] * (acc[mt][e] * (BITS == 4 ? 0.0625f : 1.0f));
             }
     }
 }
@@ -498,7 +516,7 @@ int launch(float *y, const int8_t *xq, const float *x_scale, const void *wq, int
     if (ksplit > nsb) ksplit = nsb;
     const int warps = tpc * ksplit;
     const int grid = (tiles + tpc - 1) / tpc;
-    const size_t fixed = (size_t)8 * MT * (k + 16) + ((size_t)warps * 8 + MAX_WARPS) * sizeof(uint64_t);
+    const size_t fixed = (size_t)8 * MT * (k + 16) + ((size_t)warps * 8 + MAX_WARPS) * sizeof(uint64_t) + 16 * sizeof(float);
     if (fixed + (size_t)warps * 2 * UNIT_BYTES > smem_cap)  // activations of a very long k leave no room for the rings
         return launch_tile<MT, DUMP, BITS>(y, xq, x_scale, wq, m, n, k, partials, st);
     const int per_warp = (nsb + ksplit - 1) / ksplit;
