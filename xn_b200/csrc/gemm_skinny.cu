@@ -217,7 +217,12 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
         }
         T *y = static_cast<T *>(args.y) + (size_t)g * args.y_bs + ch0;
         const bool vec = left >= 4 && (args.ldy & 3) == 0 && (args.y_bs & 3) == 0 && (reinterpret_cast<uintptr_t>(args.y) & 7) == 0;
-        for (int lc = warp - 2, row = lc * S + rank; row < args.M && left > 0; lc += 4, row = lc * S + rank) {
+        // the warp's row scales (at most 32), one lane each: asked for together, not row by row between the stores
+        const int row_l = (warp - 2 + 4 * lane) * S + rank;
+        const float xs_l = F8 && row_l < args.M ? ld_act_f32(args.x_scale + row_l) : 1.0f;
+        for (int i = 0, lc = warp - 2, row = lc * S + rank; row < args.M; ++i, lc += 4, row = lc * S + rank) {
+            const float xs = F8 ? __shfl_sync(0xffffffffu, xs_l, i) : 1.0f;
+            if (left <= 0) continue;
             float4 sum = *reinterpret_cast<const float4 *>(red + (size_t)lc * BM + 4 * lane);
             for (int src = 1; src < S; ++src) {
                 const float4 p = *reinterpret_cast<const float4 *>(red + (size_t)(src * per + lc) * BM + 4 * lane);
@@ -225,7 +230,6 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             }
             float val[4] = {sum.x, sum.y, sum.z, sum.w};
             T out[4];
-            const float xs = F8 ? ld_act_f32(args.x_scale + row) : 1.0f;
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 out[i] = from_f32<T>(F8 ? ws[i] * (xs * val[i]) : val[i]);
