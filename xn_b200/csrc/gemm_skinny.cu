@@ -259,6 +259,15 @@ struct SkinnyCall {
     bool w_static;
 };
 
+// CTAs in clusters of S that are on the machine at once, two or one per SM.  A cluster has to fit a GPC: of 148 SMs' 296 / 148
+// places the driver's occupancy query gives clusters of two all, of four 284 / 132, of eight 264 / 120.  Past that the last
+// clusters are a second round: one per SM, 36 tiles in clusters of four (144 CTAs), e4m3 94 x 4608 x 1408, 16.3 us against 10.3.
+inline long long cluster_places(int S, bool two) {
+    const long long sms = sm_count();
+    if (two) return sms * 7 / 4;
+    return S <= 2 ? sms : (S <= 4 ? sms * 8 / 9 : sms * 13 / 16);
+}
+
 template <int KIND, bool MN>
 int launch(const SkinnyCall &c, cudaStream_t st) {
     constexpr int ELEM = KIND == 0 ? 1 : 2, BK = BKB / ELEM;
@@ -273,8 +282,8 @@ int launch(const SkinnyCall &c, cudaStream_t st) {
     const int num_kb = (int)((c.k + BK - 1) / BK), sms = sm_count();
     const long long units = (long long)a.tiles * (long long)c.batch;
     const int stage = BM * BKB + a.np * a.MB * BKB;
-    // The most ranges of k (a power of two: clusters of 3, 5, ... pack badly) whose CTAs all find a place at once --
-    // somewhat below two per SM, because a cluster has to fit a GPC -- with two stages each at least.  e4m3, 32 rows, us
+    // The most ranges of k (a power of two: clusters of 3, 5, ... pack badly) whose CTAs all find a place at once, with two
+    // stages each at least.  e4m3, 32 rows, us
     // for S = 1 / 2 / 4 / 8: 4096 x 4096 14.2 / 10.9 / 7.9 / 8.2; 8192 x 4096 14.8 / 12.1 / 10.5 / 16.4; 12288 x 4096
     // 15.5 / 14.6 / 17.9 / 22.9; 22528 x 4096 19.9 / 28.4 / 30.3 / 41.7; 4096 x 11264 30.8 / 21.3 / 13.8 / 12.5.
     // Half an SM's shared memory per CTA when that holds three stages beside the received partials (two, when the units
@@ -288,7 +297,7 @@ int launch(const SkinnyCall &c, cudaStream_t st) {
     // layers), at one stream eight (272 against 288).
     const int most = a.MB <= 16 || units * 6 <= sms ? 8 : 4;
     int S = 1;
-    while (S < most && units * S * 2 <= (two ? sms * 7 / 4 : sms) && num_kb / (S * 2) >= 2) S *= 2;
+    while (S < most && units * S * 2 <= cluster_places(S * 2, two) && num_kb / (S * 2) >= 2) S *= 2;
     const size_t red = red_bytes(S);
     const int nstage = (int)(((two ? half : 2 * half) - 1024 - red) / stage);
     a.nstage = nstage > SK_MAX_STAGES ? SK_MAX_STAGES : nstage;
