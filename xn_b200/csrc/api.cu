@@ -119,7 +119,7 @@ static int gemm_dispatch(xn_dtype dtype, void *dst, const void *lhs, size_t lhs_
     // us, streaming / tensor memory, bf16: 1 x 4096 x 4096 8.0 / 8.9, 1 x 22528 x 4096 28.3 / 31.0, 1 x 4096 x 11264
     // 20.3 / 17.3; 16 x 4096 x 4096 10.7 / 9.3, 16 x 12288 x 4096 20.9 / 19.8, 16 x 22528 x 4096 31.4 / 33.4.
     const bool narrow = (n + 127) / 128 <= (size_t)sm_count();
-    const bool skinny16 = tn16_ok && lhs_b == 1 && !causal && gemm_skinny_wanted(m, n, k) &&
+    const bool skinny16 = tn16_ok && lhs_b == 1 && !causal && gemm_skinny_wanted(m, n, 2 * k, 1) &&
                           (m > 16 || !h16_fits || (n >= 256 && narrow && (m > 8 || (k >= 8192 && (n + 63) / 64 <= (size_t)sm_count()))));
     if (skinny16)
         return launch_skinny_16bit(dtype, dst, l, r, take_fused_col_bias(), m, n, k, lhs_rs, rhs_cs, dst_rs, 1, 0, 0, 0, false,
@@ -135,7 +135,7 @@ static int gemm_dispatch(xn_dtype dtype, void *dst, const void *lhs, size_t lhs_
     const bool kn16_rhs = dtype != XN_F32 && lhs_cs == 1 && rhs_cs == 1 && dst_cs == 1 && rhs_rs % 8 == 0 && rhs_rs >= n && aligned(r, 16) &&
                           (lhs_b == 1 || rhs_b_stride % 8 == 0);
     if (kn16_rhs && lhs_b == 1 && !causal && k % 8 == 0 && lhs_rs % 8 == 0 && aligned(l, 16) && dst_rs <= 0x7fffffff &&
-        gemm_skinny_wanted(m, n, k))
+        gemm_skinny_wanted(m, n, 2 * k, 1))
         return launch_skinny_16bit(dtype, dst, l, r, nullptr, m, n, k, lhs_rs, rhs_rs, dst_rs, 1, 0, 0, 0, true, (cudaStream_t)stream);
     if (kn16_rhs && m <= 16 && !causal && gemv_kn16_fits(m, n, k, lhs_b))
         return launch_gemv_kn16(dtype, dst, l, r, m, n, k, lhs_b, lhs_b_stride, rhs_b_stride, dst_rs, lhs_rs, rhs_rs,

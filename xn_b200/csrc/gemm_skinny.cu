@@ -340,13 +340,24 @@ int launch(const SkinnyCall &c, cudaStream_t st) {
 
 }  // namespace
 
-// Whether this kernel is the one for m rows against an [n, k] weight.  Up to 64 rows always (the callers know which
-// smaller row counts their weight-streaming kernels still win).  From 65 to 128 rows while the channels make at most half
-// as many tiles as there are SMs, so that k can be split: W8A16 at 96 rows, 4096 x 4096, 15.4 us tiled -> 10.9; bf16
-// 4096 x 11264 27.8 -> 24.2; with more channels 128-row tiles re-read less of x (12288 x 4096: 18.7 tiled, 19.8 here).
-bool gemm_skinny_wanted(size_t m, size_t n, size_t k) {
-    if (n > 0x7fffff00 || k > 0x7fffff00 || (n + BM - 1) / BM > 0x7fffffff / 8) return false;
-    return m <= 64 || (m <= 128 && (n + BM - 1) / BM * 2 <= (size_t)sm_count());
+// Whether this kernel is the one for m rows against a weight of n channels of k_bytes each (pieces: e4m3 matrices per activation,
+// 1 for 16-bit rows).  Up to 64 rows always (the callers know which smaller row counts their weight-streaming kernels still
+// win).  From 65 to 128 rows while the channels make at most half as many tiles as there are SMs, so that k can be split, and k is
+// long enough to pay for moving MB x 128 partial sums per CTA through the cluster, which the tiled kernel does not do: that cost
+// grows with MB^2 (rows, and columns per owner) and is paid back per k stage, twice as fast where two pieces share a weight
+// stage.  With fewer than 33 tiles the tiled kernel leaves more of the machine idle and k may be shorter.  us, tiled / this
+// kernel: bf16 66 x 4096 x 512 6.2 / 6.5, x 1024 8.8 / 7.2; 128 x 8192 x 2048 14.7 / 15.5, x 4096 23.6 / 21.4; W8A8 128 x 8192 x 1024
+// 6.9 / 10.0, 80 x 8192 x 2048 9.7 / 9.8, x 4096 14.3 / 13.1; W8A16 128 x 2048 x 1024 7.2 / 7.8, x 2048 10.3 / 8.5.
+bool gemm_skinny_wanted(size_t m, size_t n, size_t k_bytes, int pieces) {
+    if (n > 0x7fffff00 || k_bytes > 0x7fffff00 || (n + BM - 1) / BM > 0x7fffffff / 8) return false;
+    if (m <= 64) return true;
+    const size_t tiles = (n + BM - 1) / BM, mb = (m + 15) / 16 * 16, work = k_bytes * (size_t)pieces;
+    if (m > 128 || tiles * 2 > (size_t)sm_count()) return false;
+    if (tiles <= 32) {
+        const size_t line = mb * mb / 8 > 1024 ? mb * mb / 8 : 1024;
+        return pieces == 1 ? work >= line : work > line;
+    }
+    return work * 25 >= mb * mb * 8 && !(pieces == 1 && mb == 128 && k_bytes > 8192);
 }
 
 // y bf16 [m, n] = x_scale[m] * w_scale[n] * (x_hi (+ x_lo)) * wq^T, all operands row-major e4m3.  wq is a static weight.

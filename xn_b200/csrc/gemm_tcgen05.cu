@@ -1427,7 +1427,7 @@ int launch_attention_prefill(xn_dtype dt, void *out, size_t ldo, const void *q, 
 // y bf16 [m,n] = x_scale[m] * w_scale[n] * (x_hi (+ x_lo)) * wq^T, all operands row-major e4m3.
 int launch_linear_fp8_gemm(void *y, const uint8_t *x_hi, const uint8_t *x_lo, const float *x_scale, const uint8_t *wq,
                            const float *w_scale, size_t m, size_t n, size_t k, cudaStream_t st) {
-    if (gemm_skinny_wanted(m, n, k)) return launch_skinny_fp8(y, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, n, st);
+    if (gemm_skinny_wanted(m, n, k, x_lo ? 2 : 1)) return launch_skinny_fp8(y, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, n, st);
     GemmArgs a{};
     a.y[0] = y; a.ndst = 1; a.col_offset = 0; a.batch = 1; a.y_batch_stride = 0;
     a.x_scale = x_scale; a.w_scale = w_scale; a.M = (int)m; a.N = (int)n; a.K = (int)k; a.ldy = (int)n;
