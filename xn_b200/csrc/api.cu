@@ -115,12 +115,16 @@ static int gemm_dispatch(xn_dtype dtype, void *dst, const void *lhs, size_t lhs_
                          rhs_cs % 8 == 0 && aligned(l, 16) && aligned(r, 16) && m <= 0x7fffffff && n <= 0x7fffffff &&
                          k <= 0x7fffffff && dst_rs <= 0x7fffffff;
     // Up to 16 rows the mma.sync kernel streams a weight without the tensor-memory kernel's fixed cost, except where the
-    // latter's split along k pays: a long k, or 9 to 16 rows (two column groups) while the channels leave SMs to split over.
+    // latter's split along k pays: a long k, or 9 to 16 rows (two column groups) while the channels leave SMs to split over
+    // and k is no shorter than 2048 or the channels are few.
     // us, streaming / tensor memory, bf16: 1 x 4096 x 4096 8.0 / 8.9, 1 x 22528 x 4096 28.3 / 31.0, 1 x 4096 x 11264
-    // 20.3 / 17.3; 16 x 4096 x 4096 10.7 / 9.3, 16 x 12288 x 4096 20.9 / 19.8, 16 x 22528 x 4096 31.4 / 33.4.
+    // 20.3 / 17.3; 16 x 4096 x 4096 10.7 / 9.3, 16 x 12288 x 4096 20.9 / 19.8, 16 x 22528 x 4096 31.4 / 33.4; 12 x 4096 x 1024 4.5 / 5.6,
+    // 16 x 16384 x 1024 8.9 / 9.6, 12 x 2048 x 1024 4.6 / 4.0.
     const bool narrow = (n + 127) / 128 <= (size_t)sm_count();
+    const bool few = k >= 2048 || n <= 2048;  // 9 to 16 rows
     const bool skinny16 = tn16_ok && lhs_b == 1 && !causal && gemm_skinny_wanted(m, n, 2 * k, 1) &&
-                          (m > 16 || !h16_fits || (n >= 256 && narrow && (m > 8 || (k >= 8192 && (n + 63) / 64 <= (size_t)sm_count()))));
+                          (m > 16 || !h16_fits ||
+                           (n >= 256 && narrow && (m > 8 ? few : k >= 8192 && (n + 63) / 64 <= (size_t)sm_count())));
     if (skinny16)
         return launch_skinny_16bit(dtype, dst, l, r, take_fused_col_bias(), m, n, k, lhs_rs, rhs_cs, dst_rs, 1, 0, 0, 0, false,
                                    (cudaStream_t)stream);

@@ -19,9 +19,14 @@ int launch_linear_fp8_gemm_multicast(void *y_mc, size_t ldy, size_t col_offset, 
                                      const float *x_scale, const uint8_t *wq, const float *w_scale, size_t m, size_t n,
                                      size_t k, cudaStream_t st);
 
-// Below this many weight bytes the mma.sync GEMV beats the tensor-memory kernel at up to 8 rows (us, GEMV / tensor
-// memory, W8A16, one row: 1024 x 1024 2.4 / 3.3, 4096 x 4096 7.3 / 6.8, 12288 x 4096 12.8 / 12.3, 4096 x 11264 13.8 / 11.1).
-static constexpr size_t FP8_GEMV_MAX_WEIGHT = 12u << 20;
+// Up to 8 rows the mma.sync GEMV beats the tensor-memory kernel below FP8_GEMV_MAX_WEIGHT weight bytes, and with one piece per
+// activation, which is half the GEMV's work, up to k = 4096 while the weight is not among the largest.  us, GEMV / tensor memory,
+// one row: W8A16 1024 x 1024 2.4 / 3.3, 4096 x 4096 7.3 / 6.8, 12288 x 4096 12.8 / 12.3, 4096 x 11264 13.8 / 11.1; W8A8 12288 x 1024
+// 5.1 / 5.7, 12288 x 4096 11.4 / 12.5, 16384 x 4096 13.8 / 14.8, 22528 x 4096 18.5 / 17.8, 4096 x 11264 11.5 / 11.4.
+static constexpr size_t FP8_GEMV_MAX_WEIGHT = 12u << 20, FP8_GEMV_MAX_WEIGHT_ONE_PIECE = 80u << 20;
+static inline bool fp8_gemv_wanted(size_t m, size_t n, size_t k, bool two_pieces) {
+    return m <= 8 && (n * k < FP8_GEMV_MAX_WEIGHT || (!two_pieces && k <= 4096 && n * k < FP8_GEMV_MAX_WEIGHT_ONE_PIECE));
+}
 
 static inline size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 }  // namespace xn
@@ -39,9 +44,9 @@ extern "C" int xn_mm_linear_fp8_pieces(void *y_bf16, const uint8_t *x_hi, const 
     XN_REQUIRE(aligned(wq, 16) && aligned(x_hi, 16) && (!x_lo || aligned(x_lo, 16)),
                "linear_fp8: weights and activation pieces must be 16-byte aligned");
     cudaStream_t st = (cudaStream_t)stream;
-    // Up to 8 rows (one MMA column group) of a weight too small to be worth a cluster split stream through the GEMV kernel;
+    // Up to 8 rows (one MMA column group) of a weight that is not worth a cluster split stream through the GEMV kernel;
     // anything larger goes to the tensor-memory kernels.
-    if (m <= 8 && n * k < FP8_GEMV_MAX_WEIGHT)
+    if (fp8_gemv_wanted(m, n, k, x_lo != nullptr))
         return launch_linear_fp8_gemv(y_bf16, x_hi, x_lo, x_scale, wq, w_scale, (int)m, n, (int)k, st);
     return launch_linear_fp8_gemm(y_bf16, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st);
 }
