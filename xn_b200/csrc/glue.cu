@@ -363,65 +363,70 @@ bool launch_silu_mul_vec(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T
     return false;
 }
 
-// The row in registers, one CTA per row, one read and one write: max-subtract, exp rounded to T, f32 sum of the rounded
-// values, divide.  A row may start anywhere (a context has whatever length it has): the 128-bit loads cover the
-// aligned middle of the row, the first threads take the up to 2 (V - 1) elements before and behind it.  The one-warp
-// form below, which this replaces up to 8192 16-bit (4096 f32) columns, walked the row three times through the cache:
-// 21.7 us for 256 rows of 1501, now 2.4 us.
-template <typename T, int VPT>
+// The row in registers, one read and one write: max-subtract, exp rounded to T, f32 sum of the rounded values, divide.  A
+// row may start anywhere (a context has whatever length it has): the 128-bit loads cover the aligned middle of the row, the first
+// threads take the up to 2 (V - 1) elements before and behind it; V = 1, for rows that give a lane few elements, loads them
+// one by one, so that all lanes share the exponentials.  WARP: a warp per row and several rows per CTA, for short rows; otherwise
+// a CTA per row.  Lines and figures: see the launcher.
+template <typename T, int VPT, bool WARP, int V = 16 / (int)sizeof(T)>
 __global__ void __launch_bounds__(256)
-softmax_row_kernel(T *dst, const T *src, int cols) {
-    constexpr int V = 16 / (int)sizeof(T);
-    __shared__ float red[32];
+softmax_row_kernel(T *dst, const T *src, size_t rows, int cols) {
+    __shared__ float red[WARP ? 1 : 32];
     dependent_begin<false>();
-    const size_t row = blockIdx.x;
+    const size_t row = WARP ? (size_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.x;
+    if (WARP && row >= rows) return;  // whole warps
+    const int tx = WARP ? (int)threadIdx.x & 31 : (int)threadIdx.x, nt = WARP ? 32 : (int)blockDim.x;
     const T *x = src + row * cols;
     T *y = dst + row * cols;
-    const int head = min(cols, (int)(((16 - (reinterpret_cast<uintptr_t>(x) & 15)) & 15) / sizeof(T)));
+    const int head = V == 1 ? 0 : min(cols, (int)(((16 - (reinterpret_cast<uintptr_t>(x) & 15)) & 15) / sizeof(T)));
     const int nvec = (cols - head) / V, tail0 = head + nvec * V;
     // edge element of this thread: the first V lie before the middle, the next V behind it
-    const int e = threadIdx.x < (unsigned)V ? (int)threadIdx.x : tail0 + (int)threadIdx.x - V;
-    const bool edge = threadIdx.x < (unsigned)V ? e < head : (threadIdx.x < 2u * V && e < cols);
+    const int e = tx < V ? tx : tail0 + tx - V;
+    const bool edge = V > 1 && (tx < V ? e < head : (tx < 2 * V && e < cols));
     float ev = edge ? to_f32(ld_act(x + e)) : -INFINITY, v[VPT][V];
     float mx = ev;
     const uint4 *xv = reinterpret_cast<const uint4 *>(x + head);
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
-        const int idx = u * (int)blockDim.x + (int)threadIdx.x;
+        const int idx = u * nt + tx;
         if (idx < nvec) {
-            const uint4 q = ld_act128(xv + idx);
+            uint4 q;
+            if constexpr (V == 1) *reinterpret_cast<T *>(&q) = ld_act(x + idx);
+            else q = ld_act128(xv + idx);
             const T *el = reinterpret_cast<const T *>(&q);
 #pragma unroll
             for (int j = 0; j < V; ++j) mx = fmaxf(mx, v[u][j] = to_f32(el[j]));
         }
     }
-    mx = block_max2(mx, red);
+    mx = WARP ? warp_max(mx) : block_max2(mx, red);
     // the reference subtracts in the element type: (x - max) is rounded before the exponential
     auto ex = [&](float a) { return to_f32(from_f32<T>(expf(to_f32(from_f32<T>(a - mx))))); };
     float sum = 0.0f;
     if (edge) sum = ev = ex(ev);
 #pragma unroll
     for (int u = 0; u < VPT; ++u)
-        if (u * (int)blockDim.x + (int)threadIdx.x < nvec)
+        if (u * nt + tx < nvec)
 #pragma unroll
             for (int j = 0; j < V; ++j) sum += v[u][j] = ex(v[u][j]);
-    sum = block_sum(sum, red);
+    sum = WARP ? warp_sum(sum) : block_sum(sum, red);
     if (edge) y[e] = from_f32<T>(ev / sum);
     uint4 *yv = reinterpret_cast<uint4 *>(y + head);
 #pragma unroll
     for (int u = 0; u < VPT; ++u) {
-        const int idx = u * (int)blockDim.x + (int)threadIdx.x;
+        const int idx = u * nt + tx;
         if (idx < nvec) {
             uint4 q;
             T *el = reinterpret_cast<T *>(&q);
 #pragma unroll
             for (int j = 0; j < V; ++j) el[j] = from_f32<T>(v[u][j] / sum);
-            yv[idx] = q;
+            if constexpr (V == 1) y[idx] = *el;
+            else yv[idx] = q;
         }
     }
 }
 
-// Rows too long for the registers of a CTA, or src and dst at different offsets from a 16-byte boundary.
+// Rows too long for the registers of a CTA, or src and dst at different offsets from a 16-byte boundary: three walks of the row
+// through the cache (256 rows of 1501 bf16 21.7 us, 2.4 with the row in registers).
 // One warp per row: max-subtract, exp rounded to T, f32 sum of the rounded values, divide.
 template <typename T>
 __global__ void softmax_kernel(T *__restrict__ dst, const T *__restrict__ src, size_t rows, size_t cols) {
@@ -1178,10 +1183,26 @@ extern "C" int xn_mm_softmax(xn_dtype dtype, void *dst, const void *src, size_t 
     XN_REQUIRE(blocks <= 0x7fffffffull, "softmax: too many rows");
     const size_t nvec = cols * dtype_size(dtype) / 16;
     if (nvec <= 1024 && rows <= 0x7fffffffull && (reinterpret_cast<uintptr_t>(dst) ^ reinterpret_cast<uintptr_t>(src)) % 16 == 0) {
-        const unsigned nt = nvec >= 256 ? 256 : (nvec < 32 ? 32 : (unsigned)(nvec + 31) / 32 * 32);
+        // A warp per row up to 256 elements, and up to 512 where the rows are many (a row with a CTA of its own costs 0.55 ns of
+        // launching, however short); single elements while a lane gets at most four 16-bit or two f32 ones.  65536 rows, us, CTA
+        // per row / one-warp form below / this: bf16 of 32 columns 36.2 / 17.0 / 8.0, of 64 36.3 / 21.1 / 10.5, of 257 40.2 / 162 /
+        // 27.0; f32 of 64 36.0 / 22.7 / 11.5, of 256 36.3 / 29.5 / 23.5.
+        const bool single = cols <= (dtype == XN_F32 ? 64 : 128);
+        const size_t most = dtype == XN_F32 ? 64 : 32;  // vectors in 256 elements
+        const bool warp = single || nvec <= most || (nvec <= 2 * most && rows >= (size_t)sm_count() * 64);
+        // rows per CTA: eight once that gives every SM one, else two
+        const unsigned per = warp ? (rows >= (size_t)sm_count() * 8 ? 8 : 2) : 1;
+        const unsigned nt = warp ? per * 32 : (nvec >= 256 ? 256 : (unsigned)(nvec + 31) / 32 * 32);
+        const dim3 grid((unsigned)((rows + per - 1) / per));
         XN_DISPATCH_DTYPE(dtype, T, {
-            auto kern = nvec <= 256 ? softmax_row_kernel<T, 1> : (nvec <= 512 ? softmax_row_kernel<T, 2> : softmax_row_kernel<T, 4>);
-            return launch_dependent(kern, dim3((unsigned)rows), dim3(nt), 0, (cudaStream_t)stream, (T *)dst, (const T *)src, (int)cols);
+            auto kern = single ? (cols <= 32 ? softmax_row_kernel<T, 1, true, 1>
+                                             : (cols <= 64 ? softmax_row_kernel<T, 2, true, 1> : softmax_row_kernel<T, 4, true, 1>))
+                        : warp ? (nvec <= 32   ? softmax_row_kernel<T, 1, true>
+                                  : nvec <= 64 ? softmax_row_kernel<T, 2, true>
+                                               : softmax_row_kernel<T, 4, true>)
+                               : (nvec <= 256 ? softmax_row_kernel<T, 1, false>
+                                              : (nvec <= 512 ? softmax_row_kernel<T, 2, false> : softmax_row_kernel<T, 4, false>));
+            return launch_dependent(kern, grid, dim3(nt), 0, (cudaStream_t)stream, (T *)dst, (const T *)src, rows, (int)cols);
         });
     }
     XN_DISPATCH_DTYPE(dtype, T, softmax_kernel<T><<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
