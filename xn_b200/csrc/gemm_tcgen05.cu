@@ -1185,6 +1185,17 @@ inline double tile_rounds(long long tiles, int num_kb, int na, bool may_cut) {
     if (parts <= 1) return (double)((tiles + sms - 1) / sms);
     return (double)(tiles / sms) + 1.0 / (double)parts + (double)tail_stages(na) / num_kb;
 }
+// Cost of a tile width: k stages of the busiest SM times the rows it pulls per stage, and what a cut costs in the same unit.
+// Behind full rounds that is the stages above; where every tile is cut the records of a narrow tile are smaller and the price
+// is their bytes: fitted to 45 products of 129 to 640 rows at seven widths, about 0.5 us and 0.4 us per MB.  (With the stages
+// for both, narrow tiles looked too cheap or too dear by turns: bf16 256 x 4096 x 11264 took three ranges of 192 columns, 36.4 us,
+// against 34.3 with two of 128; W8A8 300 x 2048 x 8192 18.7 uncut against 16.5.)
+inline double tile_cost(long long tiles, int num_kb, int na, bool may_cut, int bn) {
+    const long long sms = sm_count(), parts = may_cut ? tail_parts(tiles, num_kb, na) : 1, rows = na * BM + bn;
+    if (parts <= 1 || tiles > sms) return tile_rounds(tiles, num_kb, na, may_cut) * num_kb * (double)rows;
+    const double record_mb = (double)(tiles * parts) * bn * BM * sizeof(float) / 1e6;
+    return (double)((num_kb + parts - 1) / parts * rows) + 1000.0 + 375.0 * record_mb;
+}
 // A captured launch may be replayed beside anything: it takes no scratch it would share.  Peers' buffers stay with
 // the tiled kernel's own epilogue.
 inline bool may_cut_tail(const GemmArgs &a, cudaStream_t st) {
@@ -1296,7 +1307,7 @@ int launch_kind(const void *a0, const void *a1, const void *b, size_t lda, size_
     const int bn_step = args.b_mn ? 64 : 32;  // an n-contiguous B arrives in 64-column blocks
     for (int bn = 256; bn >= 64; bn -= bn_step) {
         const long long tiles = m_tiles * ((args.N + bn - 1) / bn);
-        const double cost = tile_rounds(tiles, num_kb, NA, may_cut) * (NA * BM + bn);
+        const double cost = tile_cost(tiles, num_kb, NA, may_cut, bn);
         if (best_cost < 0 || cost < best_cost) { best_cost = cost; best = bn; }
     }
     if (force_bn >= 64 && force_bn <= 256 && force_bn % bn_step == 0) best = force_bn;
