@@ -123,6 +123,16 @@ int wait_ctx(WaitCtx *out) {
     return XN_OK;
 }
 
+// A block that has to grow grows by half at least: what is retired on the way (kept until xn_mm_release_scratch) stays below
+// twice the block in use, also where every call wants a little more than the one before -- p.v over a growing context.
+static size_t grown(size_t have, size_t want) { return have + have / 2 > want ? have + have / 2 : want; }
+static int scratch_alloc(void **p, size_t bytes) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaSuccess) return XN_OK;
+    cudaGetLastError();
+    return fail(XN_ERR_CUDA, "library scratch of %zu bytes: %s", bytes, cudaGetErrorString(e));
+}
+
 // Scratch of the skinny path (partial accumulators + arrival counters) and of the f32 repack: one buffer per
 // (device, stream), allocated when a stream first needs it and replaced by a larger one on demand.  Calls on one
 // stream are ordered, so they can share; calls on different streams get different buffers and may overlap.
@@ -161,15 +171,21 @@ int skinny_scratch(cudaStream_t st, size_t partial_bytes, size_t ncounters, Skin
     }
     SkinnyScratch &s = e->s;
     if (s.partial_bytes < partial_bytes) {
+        size_t bytes = grown(s.partial_bytes, partial_bytes);
         void *p = nullptr;
-        XN_CHECK_CUDA(cudaMalloc(&p, partial_bytes));
+        if (cudaMalloc(&p, bytes) != cudaSuccess) {
+            cudaGetLastError();  // not left for a later launch's check to find
+            bytes = partial_bytes;
+            if (int rc = scratch_alloc(&p, bytes)) return rc;
+        }
         if (s.partials) g_retired.push_back(Retired{dev, s.partials});
         s.partials = static_cast<float *>(p);
-        s.partial_bytes = partial_bytes;
+        s.partial_bytes = bytes;
     }
     if (s.ncounters < ncounters) {
+        ncounters = grown(s.ncounters, ncounters);
         void *p = nullptr;
-        XN_CHECK_CUDA(cudaMalloc(&p, ncounters * sizeof(unsigned)));
+        if (int rc = scratch_alloc(&p, ncounters * sizeof(unsigned))) return rc;
         // the counters must read zero before the first launch that uses them: ordered on the caller's stream
         XN_CHECK_CUDA(cudaMemsetAsync(p, 0, ncounters * sizeof(unsigned), st));
         if (s.counters) g_retired.push_back(Retired{dev, s.counters});
