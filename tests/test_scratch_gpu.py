@@ -26,3 +26,38 @@ def test_a_growing_context_does_not_pile_up_scratch(xn, cuda):
     ref = p[..., :hi - 1].double() @ v[:, :hi - 1].double()
     assert bool(((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 0.02).all())
     xn._lib.check(xn.lib().xn_mm_release_scratch(None, 1))
+
+
+def test_rows_off_16_byte_boundaries_under_capture(xn, cuda):
+    """The first call of its kind may be a captured one: it takes no scratch."""
+    xn._lib.check(xn.lib().xn_mm_release_scratch(None, 1))
+    g = torch.Generator(device=cuda).manual_seed(2)
+    x = torch.randn(3, 70, 1003, generator=g, device=cuda).bfloat16()
+    w = torch.randn(3, 1003, 72, generator=g, device=cuda).bfloat16()
+    y = torch.zeros(3, 70, 72, device=cuda, dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        xn.matmul_(y, x, w, False)
+    for _ in range(2):
+        y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        ref, mag = x.double() @ w.double(), x.double().abs() @ w.double().abs()
+        assert bool(((y.double() - ref).abs() <= 2.0 ** -8 * ref.abs() + 1003 * 2.0 ** -24 * mag).all())
+
+
+def test_rows_too_many_to_be_copied(xn, cuda):
+    """Above half a GB of rows the any-stride kernel takes the product."""
+    m, n, k = 1 << 17, 8, 2049
+    x = torch.randint(-2, 3, (m, k), device=cuda, dtype=torch.int8).half()
+    w = torch.randint(-2, 3, (k, n), device=cuda, dtype=torch.int8).half()
+    xn._lib.check(xn.lib().xn_mm_release_scratch(None, 1))
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    y = torch.empty(m, n, device=cuda, dtype=torch.float16)
+    xn.matmul_(y, x, w, False)
+    torch.cuda.synchronize()
+    assert free0 - torch.cuda.mem_get_info()[0] < 64 << 20
+    for r in (slice(0, 64), slice(m - 64, m)):  # sums of small integers: exact in f32, one rounding to f16
+        assert torch.equal(y[r], (x[r].double() @ w.double()).half())

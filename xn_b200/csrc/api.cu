@@ -199,13 +199,16 @@ static int gemm_dispatch(xn_dtype dtype, void *dst, const void *lhs, size_t lhs_
                                        (rhs_b_stride >= k * rhs_rs || (rhs_b_stride >= n && lhs_b * rhs_b_stride <= rhs_rs)))))
             return launch_gemm_kn_16bit(dtype, dst, l, r, m, n, k, lhs_rs, rhs_rs, dst_rs, lhs_b, lhs_b_stride, rhs_b_stride,
                                         (cudaStream_t)stream, causal == 2 ? 2 : 0, causal_off);
-        // rows of lhs off 16-byte boundaries: copied to a pitch TMA can address first
+        // rows of lhs off 16-byte boundaries: copied to a pitch TMA can address first, where there is scratch for it
         const size_t most = (size_t)1 << 30;
         if (!kn_off && kn16_rhs && !causal && (k % 8 || lhs_rs % 8 || lhs_b_stride % 8 || !aligned(l, 16)) && n >= 2 && m <= most && n <= most &&
             k <= most && dst_rs <= 0x7fffffff && lhs_b <= 0x7fffffff &&
-            (lhs_b == 1 || rhs_b_stride >= k * rhs_rs || (rhs_b_stride >= n && lhs_b * rhs_b_stride <= rhs_rs)))
-            return launch_gemm_kn_repitched(dtype, dst, l, r, m, n, k, lhs_b, lhs_b_stride, rhs_b_stride, dst_rs, lhs_rs, rhs_rs,
-                                            (cudaStream_t)stream);
+            (lhs_b == 1 || rhs_b_stride >= k * rhs_rs || (rhs_b_stride >= n && lhs_b * rhs_b_stride <= rhs_rs))) {
+            bool taken = false;
+            const int rc = launch_gemm_kn_repitched(dtype, dst, l, r, m, n, k, lhs_b, lhs_b_stride, rhs_b_stride, dst_rs, lhs_rs, rhs_rs,
+                                                    (cudaStream_t)stream, &taken);
+            if (rc || taken) return rc;
+        }
     }
     if (causal == 2)
         return fail(XN_ERR_UNSUPPORTED, "gemm_causal (values): needs 16-bit elements, an n-contiguous right-hand side and "

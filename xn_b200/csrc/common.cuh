@@ -195,7 +195,7 @@ bool gemv_kn16_fits(size_t m, size_t n, size_t k, size_t batch);
 int launch_gemv_kn16(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k, size_t batch,
                      size_t lhs_bs, size_t rhs_bs, size_t dst_rs, size_t lhs_rs, size_t rhs_rs, cudaStream_t st);
 int launch_gemm_kn_repitched(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k, size_t batch,
-                             size_t lhs_bs, size_t rhs_bs, size_t dst_rs, size_t lhs_rs, size_t rhs_rs, cudaStream_t st);
+                             size_t lhs_bs, size_t rhs_bs, size_t dst_rs, size_t lhs_rs, size_t rhs_rs, cudaStream_t st, bool *taken);
 int launch_gemv_f32x3(float *dst, const float *lhs, const float *rhs, size_t m, size_t n, size_t k, size_t dst_rs,
                       size_t lhs_rs, size_t rhs_cs, cudaStream_t st);
 int launch_gemv_dense(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k,
