@@ -138,7 +138,9 @@ __device__ __forceinline__ uint4 ldg_stream(const void *p) {
 // Kernels launched with launch_dependent() start with this: nothing is touched before the previous kernel in the stream
 // has finished.  EARLY lets the next kernel begin its own set-up, and fetch what is static (a linear's weights above all),
 // while this one runs.  That is for outputs nobody uses as a weight (quantized pieces, caches, attention rows): a tensor
-// a caller may hand to a Linear as its weight right away (a sum, a normalised or softmaxed matrix) is written without it.
+// a caller may hand to a Linear as its weight right away (a sum, a normalised or softmaxed matrix, the product of a few rows) is
+// written without it.  The many-row and cluster matmuls announce themselves for all their callers, as xn_mm.h's promise on
+// `weight` lets them: without it a bf16 matmul of 32 x 11264 x 2048 takes 14.3 us instead of 13.0.
 template <bool EARLY = true> __device__ __forceinline__ void dependent_begin() {
     if (EARLY) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -228,8 +228,7 @@ gemv_h16_batched_kernel(T *__restrict__ y, const T *__restrict__ x, const T *__r
     const int ks = warp & (ksplit - 1), tw = warp / ksplit, tstep = BH_WARPS / ksplit;
     const int nst = (k + 31) / 32, units = (nst + BH_UNIT - 1) / BH_UNIT;
     const int u0 = units * ks / ksplit, u1 = units * (ks + 1) / ksplit;
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    dependent_begin<false>();
 
     for (int b = blockIdx.y; b < batches; b += gridDim.y) {
         const T *X = x + (size_t)b * xb, *W = w + (size_t)b * wb;

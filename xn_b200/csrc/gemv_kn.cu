@@ -69,7 +69,7 @@ gemv_kn16_kernel(T *__restrict__ y, const T *__restrict__ x, const T *__restrict
     // cw (1 or 2) strips of 64 columns per CTA, kw warps along k per strip
     const int kw = KN_WARPS / cw, wk = warp & (kw - 1), wc = warp / kw;
     const int b = (int)(strip_id / strips), j0 = ((int)(strip_id - (long long)b * strips) * cw + wc) * KN_COLS;
-    dependent_begin();
+    dependent_begin<false>();
 
     const T *X = x + (size_t)b * xb;
     const int col = j0 + 8 * g;                       // this lane's 8 output columns
