@@ -153,6 +153,13 @@ __device__ __forceinline__ uint4 ld_act128(const void *p) {
     asm volatile("ld.global.cg.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
     return v;
 }
+// The same for what every CTA reads: an ordinary load, which sees what the wait made visible and which L1 serves to the next
+// CTA of the SM.  The compiler may move it, so the pointer is to be made anew behind the wait (asm volatile("" : "+l"(p))).
+__device__ __forceinline__ uint4 ld128(const uint4 *p) {
+    uint4 v;
+    asm("ld.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
 __device__ __forceinline__ float ld_act_f32(const float *p) {
     float v;
     asm volatile("ld.global.cg.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");

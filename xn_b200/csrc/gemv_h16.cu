@@ -129,6 +129,12 @@ gemv_h16_kernel(T *__restrict__ y, const T *__restrict__ x, const T *__restrict_
     }
 
     // fixed-order reduction over the ksplit warps of a tile, then the store
+    // the bias follows the stream order like the activations (the weight alone does not): read behind the wait
+    float bs[2] = {0.0f, 0.0f};
+    if (bias && ks == 0 && valid)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if ((size_t)tile * 16 + g + 8 * h < n) bs[h] = to_f32(ld_act(bias + (size_t)tile * 16 + g + 8 * h));
     if (ksplit > 1) {
         if (ks > 0)
 #pragma unroll
@@ -152,7 +158,7 @@ gemv_h16_kernel(T *__restrict__ y, const T *__restrict__ x, const T *__restrict_
                 const int row_m = 8 * mt + 2 * t + (i & 1);
                 if (row_n < n && row_m < m) {
                     T v = from_f32<T>(acc[mt][i]);
-                    if (bias) v = from_f32<T>(to_f32(v) + to_f32(bias[row_n]));  // nn::Linear: added to the rounded product
+                    if (bias) v = from_f32<T>(to_f32(v) + bs[i >> 1]);  // nn::Linear: added to the rounded product
                     y[(size_t)row_m * ldy + row_n] = v;
                 }
             }

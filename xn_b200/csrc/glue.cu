@@ -193,10 +193,11 @@ __device__ __forceinline__ float block_max_once(float v, float *red) {
 // per element are the other half of it.
 template <typename T, int VPT, bool SPLIT>
 __global__ void __launch_bounds__(NTV)
-rms_norm_vec_kernel(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T *src, const T *__restrict__ alpha, int cols, float eps,
-                    const T *res, T *sum_out) {
+rms_norm_vec_kernel(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T *src, const T *alpha, int cols, float eps, const T *res,
+                    T *sum_out) {
     __shared__ float red[2][32];
     dependent_begin<SPLIT>();
+    asm volatile("" : "+l"(alpha));  // may be what the previous kernel wrote: no load of it is moved ahead of the wait
     const size_t row = blockIdx.x, base = row * (size_t)cols;
     const int nvec = cols / 8;
     uint4 v[VPT], r[VPT];
@@ -245,7 +246,7 @@ rms_norm_vec_kernel(T *dst, uint8_t *hi, uint8_t *lo, float *scale, const T *src
     for (int i = 0; i < VPT; ++i) {
         const int idx = i * (int)blockDim.x + (int)threadIdx.x;
         if (idx >= nvec) continue;
-        const uint4 al = __ldg(reinterpret_cast<const uint4 *>(alpha) + idx);
+        const uint4 al = ld128(reinterpret_cast<const uint4 *>(alpha) + idx);
         unsigned *w = reinterpret_cast<unsigned *>(&v[i]);
         const unsigned *q = reinterpret_cast<const unsigned *>(&al);
 #pragma unroll
