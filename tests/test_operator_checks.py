@@ -46,3 +46,12 @@ def test_int4_layer_takes_any_leading_dimensions(xn, cuda, shape):
     if x.numel():
         xq, xs = xn.quantize_rows_i8(x.reshape(-1, 256))
         assert torch.equal(y.reshape(-1, 48), xn.linear_q4(xq, xs, layer.wq, 48))
+
+
+@pytest.mark.gpu
+def test_add_of_transposed_views(xn, cuda):
+    a, b = torch.randn(37, 50, device=cuda), torch.randn(37, 50, device=cuda)
+    for x, y in ((a.t(), b.t()), (a.t(), b.t().contiguous()), (a.t().contiguous(), b.t())):
+        assert torch.equal(xn.ops.add(x, y), x + y)
+    with pytest.raises(xn.XnError):
+        xn.ops.add(a, b[:5])

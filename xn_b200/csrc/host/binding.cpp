@@ -11,7 +11,6 @@
 
 #include <ATen/core/Tensor.h>
 #include <ATen/cuda/EmptyTensor.h>
-#include <ATen/ops/empty_like.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/python_variable.h>
 
@@ -421,7 +420,9 @@ XN_BINDING(add, 2) {
     const at::Tensor &x = tensor(a[0]), &y = tensor(a[1]);
     require_cuda(x);
     require_cuda(y);
-    at::Tensor out = at::empty_like(x);
+    if (x.numel() != y.numel() || x.scalar_type() != y.scalar_type())
+        raise_xn(XN_ERR_INVALID, "add expects two tensors of one shape and type, got %s and %s", shape_text(x).c_str(), shape_text(y).c_str());
+    at::Tensor out = empty(x.sizes(), x.scalar_type(), x.device());  // contiguous, like the copies it is written from
     const at::Tensor xc = x.contiguous(), yc = y.contiguous();
     const xn_dtype dt = dtype_code(x.scalar_type());
     void *o = out.data_ptr(), *st = stream();
