@@ -1,5 +1,5 @@
-"""What the library keeps for itself, and what happens when there is none of it: a context that grows by one key per call, a first call
-under capture, an operand too large to be copied."""
+"""What the library keeps for itself: a context that grows by one key per call, a first call under capture, an operand too large to be
+copied."""
 import pytest
 import torch
 
@@ -29,7 +29,7 @@ def test_a_growing_context_does_not_pile_up_scratch(xn, cuda):
 
 
 def test_rows_off_16_byte_boundaries_under_capture(xn, cuda):
-    """The first call of its kind may be a captured one: it takes no scratch."""
+    """The first call of its kind may be a captured one."""
     xn._lib.check(xn.lib().xn_mm_release_scratch(None, 1))
     g = torch.Generator(device=cuda).manual_seed(2)
     x = torch.randn(3, 70, 1003, generator=g, device=cuda).bfloat16()

@@ -246,6 +246,8 @@ constexpr int SCRATCH_MAIN = 0;  // operands repacked for a launch, split sums
 constexpr int SCRATCH_TAIL = 1;  // the tiled kernel's records of cut tiles: its operands may lie in the other buffer
 int skinny_scratch(cudaStream_t st, size_t partial_bytes, size_t ncounters, SkinnyScratch *out, int slot = SCRATCH_MAIN);
 int library_scratch(cudaStream_t st, size_t bytes, void **out);
+// The same for launches that may be captured cold: under capture a block of the graph's own (runtime.cu).
+int launch_scratch(cudaStream_t st, size_t bytes, int slot, void **out);
 // Held by a call that hands data from one of its launches to the next through library scratch, from the lookup to the last
 // launch: another host thread's call on the same stream must not enqueue between them and overwrite the scratch.  One lock
 // per (device, stream), so a thread whose launch blocks on a full queue holds up nobody else's stream; recursive, because

@@ -1196,13 +1196,8 @@ inline double tile_cost(long long tiles, int num_kb, int na, bool may_cut, int b
     const double record_mb = (double)(tiles * parts) * bn * BM * sizeof(float) / 1e6;
     return (double)((num_kb + parts - 1) / parts * rows) + 1000.0 + 375.0 * record_mb;
 }
-// A captured launch may be replayed beside anything: it takes no scratch it would share.  Peers' buffers stay with
-// the tiled kernel's own epilogue.
-inline bool may_cut_tail(const GemmArgs &a, cudaStream_t st) {
-    if (a.causal || a.ndst != 1 || a.mc) return false;
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
-}
+// Peers' buffers stay with the tiled kernel's own epilogue.
+inline bool may_cut_tail(const GemmArgs &a) { return !a.causal && a.ndst == 1 && !a.mc; }
 
 template <int KIND, int BN, int NA>
 int launch_cfg(const void *a0, const void *a1, const void *b, size_t lda, size_t ldb, const GemmArgs &args,
@@ -1255,18 +1250,16 @@ int launch_cfg(const void *a0, const void *a1, const void *b, size_t lda, size_t
     const int nacc = NA == 2 && args.rows2 ? 2 : 1;
     const size_t tail = (size_t)(tiles % sms) * nacc;
     std::optional<ScratchHold> hold;  // from the records' lookup to the launch that adds them
-    if (KIND != 3 && may_cut_tail(args, st)) {
+    if (KIND != 3 && may_cut_tail(args)) {
         const int parts = tail_parts(tiles, (args.K + BKB / ELEM - 1) / (BKB / ELEM), NA);
-        SkinnyScratch sc;
+        void *records = nullptr;
         if (parts > 1) hold.emplace(st);
-        if (parts > 1 && skinny_scratch(st, tail * parts * BN * BM * sizeof(float), 0, &sc, SCRATCH_TAIL) == XN_OK) {
+        if (parts > 1 && launch_scratch(st, tail * parts * BN * BM * sizeof(float), SCRATCH_TAIL, &records) == XN_OK) {
             args2.full_tiles = (int)(tiles - tiles % sms);
             args2.tail_split = parts;
-            args2.tail_rec = sc.partials;
+            args2.tail_rec = static_cast<float *>(records);
             units = args2.full_tiles + (tiles % sms) * parts;
-        } else if (parts > 1) {
-            cudaGetLastError();  // no memory for the records: every tile is computed whole
-        }
+        }  // no memory for the records: every tile is computed whole
     }
     const int grid = (int)(units < sms ? units : sms);
     cudaLaunchConfig_t cfg = {};
@@ -1302,7 +1295,7 @@ int launch_kind(const void *a0, const void *a1, const void *b, size_t lda, size_
     const long long m_tiles = (long long)((args.M + BM - 1) / BM) * args.batch;
     int best = 256;
     double best_cost = -1;
-    const bool may_cut = KIND != 3 && may_cut_tail(args, st);
+    const bool may_cut = KIND != 3 && may_cut_tail(args);
     const int num_kb = (args.K + BKB / (KIND == 0 ? 1 : 2) - 1) / (BKB / (KIND == 0 ? 1 : 2));
     const int bn_step = args.b_mn ? 64 : 32;  // an n-contiguous B arrives in 64-column blocks
     for (int bn = 256; bn >= 64; bn -= bn_step) {

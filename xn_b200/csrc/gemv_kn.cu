@@ -304,22 +304,21 @@ int launch_gemv_kn16(xn_dtype dt, void *dst, const void *lhs, const void *rhs, s
 // (attention probabilities over a context of any length): TMA cannot address it, so its rows are copied to a pitch it
 // can, which costs one pass over m x k elements, and the tensor-memory kernel takes the product.  The map's k extent
 // stays k: what lies between k and the pitch is never read.  *taken = false, with nothing enqueued, where there is no scratch to
-// be had: under capture (a graph may be replayed beside anything, and the call may be the first of its kind), above
-// REPITCH_MAX_SCRATCH, or when the allocation fails; the caller's any-stride kernel then takes the call (32 x 100 x 128 x 1501 bf16:
-// 202 us against 19).
-constexpr size_t REPITCH_MAX_SCRATCH = (size_t)512 << 20;
+// be had -- above REPITCH_MAX_SCRATCH (REPITCH_MAX_CAPTURED for a graph, which keeps its block), or when the allocation fails;
+// the caller's any-stride kernel then takes the call (32 x 100 x 128 x 1501 bf16: 202 us against 19).
+constexpr size_t REPITCH_MAX_SCRATCH = (size_t)512 << 20, REPITCH_MAX_CAPTURED = (size_t)64 << 20;
 int launch_gemm_kn_repitched(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k, size_t batch,
                              size_t lhs_bs, size_t rhs_bs, size_t dst_rs, size_t lhs_rs, size_t rhs_rs, cudaStream_t st, bool *taken) {
     const size_t lda = (k + 7) / 8 * 8;
     *taken = false;
-    if (batch > REPITCH_MAX_SCRATCH / m || batch * m > REPITCH_MAX_SCRATCH / (lda * 2)) return XN_OK;
-    const size_t rows = batch * m;
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     XN_CHECK_CUDA(cudaStreamIsCapturing(st, &cap));
-    if (cap != cudaStreamCaptureStatusNone) return XN_OK;
+    const size_t most_bytes = cap == cudaStreamCaptureStatusNone ? REPITCH_MAX_SCRATCH : REPITCH_MAX_CAPTURED;
+    if (batch > most_bytes / m || batch * m > most_bytes / (lda * 2)) return XN_OK;
+    const size_t rows = batch * m;
     void *tmp = nullptr;
     ScratchHold hold(st);
-    if (library_scratch(st, rows * lda * 2, &tmp)) return XN_OK;
+    if (launch_scratch(st, rows * lda * 2, SCRATCH_MAIN, &tmp)) return XN_OK;
     *taken = true;
     const size_t blocks = (rows + 7) / 8, most = (size_t)sm_count() * 8;
     if (int rc = launch_dependent(repitch_rows_kernel, dim3((unsigned)(blocks < most ? blocks : most)), dim3(256), 0, st,

@@ -7,6 +7,7 @@
 // lives in pinned, mapped host memory: the host reads it without synchronising, every later launch on that
 // device is refused with XN_ERR_DEVICE until xn_mm_clear_device_status(), and xn_mm_device_status() lets a
 // caller poll it at its own synchronisation points.
+#include <list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -133,10 +134,11 @@ static int scratch_alloc(void **p, size_t bytes) {
     return fail(XN_ERR_CUDA, "library scratch of %zu bytes: %s", bytes, cudaGetErrorString(e));
 }
 
-// Scratch of the skinny path (partial accumulators + arrival counters) and of the f32 repack: one buffer per
-// (device, stream), allocated when a stream first needs it and replaced by a larger one on demand.  Calls on one
-// stream are ordered, so they can share; calls on different streams get different buffers and may overlap.
-// (xn drives a device through one stream, xn-core/src/cuda_backend.rs:52: one buffer per GPU in practice.)
+// Scratch that one launch of a call leaves for the next (repacked f32 operands, unpacked block weights, re-pitched rows; in a slot
+// of their own the records of cut tiles) and the arrival counters of the one-launch decode attention: one buffer per (device,
+// stream, slot), allocated when a stream first needs it and replaced by a larger one on demand.  Calls on one stream are
+// ordered, so they can share (ScratchHold keeps their launches together); calls on different streams get different buffers and may
+// overlap.  (xn drives a device through one stream, xn-core/src/cuda_backend.rs:52: one buffer per GPU in practice.)
 // A stream that is being captured cannot allocate: it borrows the largest buffer of its device -- the one of the
 // stream that ran the same shapes before the capture, which is how a CUDA graph is normally warmed up -- and is
 // refused with a clear message when no buffer is large enough.
@@ -196,6 +198,95 @@ int skinny_scratch(cudaStream_t st, size_t partial_bytes, size_t ncounters, Skin
     return XN_OK;
 }
 
+// Scratch of captured launches: a block per (capture, stream, use) that belongs to the graph.  A graph may be replayed beside
+// anything, so it shares no block with eager calls or other graphs; and it needs no earlier call to have left one.  The graph holds
+// the block through a user object: when the last graph and executable made of the capture are gone and their launches have
+// finished, the block is free for the next capture (xn_mm_release_scratch gives free ones back).
+namespace {
+struct GraphBlock {
+    int dev;
+    void *p;
+    size_t bytes;
+    unsigned long long capture;
+    cudaStream_t st;
+    int slot;
+    bool live;
+};
+// Never held across a CUDA call (the callback below may come from within one), never destroyed (it may come late).
+std::mutex &graph_mu() { static auto *m = new std::mutex; return *m; }
+std::list<GraphBlock> &graph_blocks() { static auto *l = new std::list<GraphBlock>; return *l; }
+void CUDART_CB graph_block_free(void *b) {
+    std::lock_guard<std::mutex> lock(graph_mu());
+    static_cast<GraphBlock *>(b)->live = false;
+}
+
+int graph_scratch(cudaStream_t st, int dev, size_t bytes, int slot, void **out) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    cudaGraph_t graph = nullptr;
+    XN_CHECK_CUDA(cudaStreamGetCaptureInfo(st, &status, &id, &graph));
+    if (status != cudaStreamCaptureStatusActive || !graph) return fail(XN_ERR_CUDA, "the capture of this stream is no longer valid");
+    size_t want = bytes;
+    GraphBlock *b = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(graph_mu());
+        for (auto &g : graph_blocks()) {
+            if (g.dev != dev) continue;
+            if (g.live && g.capture == id && g.st == st && g.slot == slot) {
+                if (g.bytes >= bytes) {
+                    *out = g.p;
+                    return XN_OK;
+                }
+                if (grown(g.bytes, bytes) > want) want = grown(g.bytes, bytes);
+            }
+            if (!g.live && g.bytes >= bytes && (!b || g.bytes < b->bytes)) b = &g;
+        }
+        if (b) {
+            b->capture = id;
+            b->st = st;
+            b->slot = slot;
+            b->live = true;
+        }
+    }
+    if (!b) {
+        void *p = nullptr;
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // an allocation is no part of the capture
+        XN_CHECK_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        const int rc = scratch_alloc(&p, want);
+        XN_CHECK_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        if (rc) return rc;
+        std::lock_guard<std::mutex> lock(graph_mu());
+        graph_blocks().push_back(GraphBlock{dev, p, want, id, st, slot, true});
+        b = &graph_blocks().back();
+    }
+    cudaUserObject_t obj = nullptr;
+    cudaError_t e = cudaUserObjectCreate(&obj, b, graph_block_free, 1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) {
+        graph_block_free(b);
+    } else if ((e = cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove)) != cudaSuccess) {
+        cudaUserObjectRelease(obj, 1);  // frees the block
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return fail(XN_ERR_CUDA, "the graph being captured does not take its scratch: %s", cudaGetErrorString(e));
+    }
+    *out = b->p;
+    return XN_OK;
+}
+}  // namespace
+
+int launch_scratch(cudaStream_t st, size_t bytes, int slot, void **out) {
+    int dev = 0;
+    if (int rc = current_device(&dev)) return rc;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    XN_CHECK_CUDA(cudaStreamIsCapturing(st, &cap));
+    if (cap != cudaStreamCaptureStatusNone) return graph_scratch(st, dev, bytes, slot, out);
+    SkinnyScratch s;
+    if (int rc = skinny_scratch(st, bytes, 0, &s, slot)) return rc;
+    *out = s.partials;
+    return XN_OK;
+}
+
 // The same per-(device, stream) buffer for other internal users (the f32 matmul's packed operands).
 int library_scratch(cudaStream_t st, size_t bytes, void **out) {
     SkinnyScratch s;
@@ -226,7 +317,7 @@ extern "C" int xn_mm_clear_device_status(void) {
     XN_CHECK_CUDA(cudaDeviceSynchronize());
     std::lock_guard<std::mutex> lock(g_mu);
     if (g_status[dev]) *g_status[dev] = 0;
-    // a launch that gave up may have left arrival counters of split tiles non-zero
+    // a launch that gave up may have left arrival counters non-zero
     for (auto &t : g_table)
         if (t.dev == dev && t.s.counters) XN_CHECK_CUDA(cudaMemset(t.s.counters, 0, t.s.ncounters * sizeof(unsigned)));
     return XN_OK;
@@ -267,6 +358,19 @@ extern "C" int xn_mm_release_scratch(void *stream, int all_streams) {
             ++i;
         }
     }
+    std::vector<void *> free_blocks;
+    {
+        std::lock_guard<std::mutex> graph_lock(graph_mu());
+        for (auto it = graph_blocks().begin(); it != graph_blocks().end();) {
+            if (it->dev == dev && !it->live) {
+                free_blocks.push_back(it->p);
+                it = graph_blocks().erase(it);
+            } else {
+                ++it;
+            }
+        }
+    }
+    for (void *p : free_blocks) XN_CHECK_CUDA(cudaFree(p));
     return XN_OK;
 }
 
