@@ -126,7 +126,7 @@ static int gemm_dispatch(xn_dtype dtype, void *dst, const void *lhs, size_t lhs_
                           (m > 16 || !h16_fits ||
                            (n >= 256 && narrow && (m > 8 ? few : k >= 8192 && (n + 63) / 64 <= (size_t)sm_count())));
     if (skinny16)
-        return launch_skinny_16bit(dtype, dst, l, r, take_fused_col_bias(), m, n, k, lhs_rs, rhs_cs, dst_rs, 1, 0, 0, 0, false,
+        return launch_skinny_16bit(dtype, dst, l, r, take_fused_col_bias(), m, n, k, lhs_rs, rhs_cs, dst_rs, false,
                                    (cudaStream_t)stream);
     if (h16_fits && lhs_b == 1 && n >= 64 && tn16_ok)
         return launch_gemv_h16(dtype, dst, l, r, m, n, k, dst_rs, lhs_rs, rhs_cs, take_fused_col_bias(), (cudaStream_t)stream);
@@ -140,7 +140,7 @@ static int gemm_dispatch(xn_dtype dtype, void *dst, const void *lhs, size_t lhs_
                           (lhs_b == 1 || rhs_b_stride % 8 == 0);
     if (kn16_rhs && lhs_b == 1 && !causal && k % 8 == 0 && lhs_rs % 8 == 0 && aligned(l, 16) && dst_rs <= 0x7fffffff &&
         gemm_skinny_wanted(m, n, 2 * k, 1))
-        return launch_skinny_16bit(dtype, dst, l, r, nullptr, m, n, k, lhs_rs, rhs_rs, dst_rs, 1, 0, 0, 0, true, (cudaStream_t)stream);
+        return launch_skinny_16bit(dtype, dst, l, r, nullptr, m, n, k, lhs_rs, rhs_rs, dst_rs, true, (cudaStream_t)stream);
     if (kn16_rhs && m <= 16 && !causal && gemv_kn16_fits(m, n, k, lhs_b))
         return launch_gemv_kn16(dtype, dst, l, r, m, n, k, lhs_b, lhs_b_stride, rhs_b_stride, dst_rs, lhs_rs, rhs_rs,
                                 (cudaStream_t)stream);

@@ -216,8 +216,7 @@ int split_rows_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_scale, const void *x,
 int launch_skinny_fp8(void *y, const uint8_t *x_hi, const uint8_t *x_lo, const float *x_scale, const uint8_t *wq,
                       const float *w_scale, size_t m, size_t n, size_t k, size_t ldy, cudaStream_t st);
 int launch_skinny_16bit(xn_dtype dt, void *dst, const void *lhs, const void *rhs, const void *bias, size_t m, size_t n, size_t k,
-                        size_t lda, size_t ldb, size_t ldd, size_t batch, size_t lhs_bs, size_t rhs_bs, size_t dst_bs, bool w_mn,
-                        cudaStream_t st);
+                        size_t lda, size_t ldb, size_t ldd, bool w_mn, cudaStream_t st);
 int launch_gemm_tn_16bit(xn_dtype dt, void *dst, const void *lhs, const void *rhs, size_t m, size_t n, size_t k,
                          size_t lda, size_t ldb, size_t ldd, size_t batch, size_t lhs_bs, size_t rhs_bs, cudaStream_t st,
                          int causal = 0, int causal_off = 0);

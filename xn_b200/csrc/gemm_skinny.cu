@@ -1,5 +1,5 @@
 // Matmul of up to 128 activation rows against a weight on the tensor cores: y[M, N] = x[M, K] * W^T with W [N, K]
-// (e4m3, bf16, f16) or W [K, N] (16-bit, n contiguous), optionally one weight per batch entry.  The decode-time linear of
+// (e4m3, bf16, f16) or W [K, N] (16-bit, n contiguous).  The decode-time linear of
 // a batch of streams (xn-core/src/nn/linear.rs:56-66), HBM-bound by the weights.
 //
 // The operands swap roles: the 128 tensor-memory lanes carry 128 output channels and the MMA's N dimension carries the
@@ -28,14 +28,11 @@ struct SkinnyArgs {
     void *y;                         // [M, ldy] bf16 (e4m3 and bf16 operands) or f16
     const float *x_scale, *w_scale;  // e4m3 operands only
     const void *bias;                // optional, 16-bit operands: added to the rounded product and rounded again
-    long long y_bs;                  // elements between the batch entries' outputs
     int ldy, M, N, K;
     int MB;      // M rounded up to 16
     int np;      // pieces per activation (1 or 2)
     int nstage;
-    int tiles;   // 128-channel tiles per batch entry
     int S;       // CTAs per cluster = ranges of k
-    int w_inner, x_inner;  // dimension order of the tensor maps (make_map3)
     int w_static;  // the weights are a model parameter: they may be fetched before the dependency wait
     WaitCtx wait;
 };
@@ -79,7 +76,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
     const int warp = warp_id(), lane = threadIdx.x & 31;
     const int S = args.S;
     const int rank = S > 1 ? (int)(blockIdx.x % (unsigned)S) : 0;  // clusters are runs of S consecutive CTAs
-    const int unit = (int)(blockIdx.x / (unsigned)S), g = unit / args.tiles, tile = unit - g * args.tiles;
+    const int tile = (int)(blockIdx.x / (unsigned)S);
     const int num_kb = (args.K + BK - 1) / BK;
     const int kb0 = num_kb * rank / S, kb1 = num_kb * (rank + 1) / S, nkb = kb1 - kb0;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -114,9 +111,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                 if (MN) {  // two blocks of 64 channels x 64 k
 #pragma unroll
                     for (int i = 0; i < 2; ++i)
-                        tma_load_3d(st + i * (64 * BKB), &map_w, tile * BM + 64 * i, args.w_inner ? g : k, args.w_inner ? k : g, bar);
+                        tma_load_3d(st + i * (64 * BKB), &map_w, tile * BM + 64 * i, k, 0, bar);
                 } else {
-                    tma_load_3d(st, &map_w, k, args.w_inner ? g : tile * BM, args.w_inner ? tile * BM : g, bar);
+                    tma_load_3d(st, &map_w, k, tile * BM, 0, bar);
                 }
             };
             const int pre = min(NSTAGE, nkb);
@@ -136,9 +133,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
                     mbar_expect_tx(&full[s], (unsigned)STAGE_BYTES);
                     load_w(it);
                 }
-                const int y = args.x_inner ? g : 0, z = args.x_inner ? 0 : g;
-                tma_load_3d(st + W_BYTES, &map_x0, k, y, z, &full[s]);
-                if (args.np == 2) tma_load_3d(st + W_BYTES + X_BYTES, &map_x1, k, y, z, &full[s]);
+                tma_load_3d(st + W_BYTES, &map_x0, k, 0, 0, &full[s]);
+                if (args.np == 2) tma_load_3d(st + W_BYTES + X_BYTES, &map_x1, k, 0, 0, &full[s]);
             }
         }
     } else if (warp == 1) {
@@ -215,8 +211,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_const
             if (F8 && i < left) ws[i] = __ldg(args.w_scale + ch0 + i);
             if (!F8 && args.bias && i < left) bs[i] = to_f32(static_cast<const T *>(args.bias)[ch0 + i]);
         }
-        T *y = static_cast<T *>(args.y) + (size_t)g * args.y_bs + ch0;
-        const bool vec = left >= 4 && (args.ldy & 3) == 0 && (args.y_bs & 3) == 0 && (reinterpret_cast<uintptr_t>(args.y) & 7) == 0;
+        T *y = static_cast<T *>(args.y) + ch0;
+        const bool vec = left >= 4 && (args.ldy & 3) == 0 && (reinterpret_cast<uintptr_t>(args.y) & 7) == 0;
         // the warp's row scales (at most 32), one lane each: asked for together, not row by row between the stores
         const int row_l = (warp - 2 + 4 * lane) * S + rank;
         const float xs_l = F8 && row_l < args.M ? ld_act_f32(args.x_scale + row_l) : 1.0f;
@@ -255,7 +251,7 @@ struct SkinnyCall {
     void *y;
     const void *x0, *x1, *w, *bias;
     const float *x_scale, *w_scale;
-    size_t m, n, k, ldx, ldw, ldy, batch, x_bs, w_bs, y_bs;
+    size_t m, n, k, ldx, ldw, ldy;
     bool w_static;
 };
 
@@ -273,14 +269,13 @@ int launch(const SkinnyCall &c, cudaStream_t st) {
     constexpr int ELEM = KIND == 0 ? 1 : 2, BK = BKB / ELEM;
     SkinnyArgs a{};
     a.y = c.y; a.x_scale = c.x_scale; a.w_scale = c.w_scale; a.bias = c.bias;
-    a.y_bs = (long long)c.y_bs; a.ldy = (int)c.ldy; a.M = (int)c.m; a.N = (int)c.n; a.K = (int)c.k;
+    a.ldy = (int)c.ldy; a.M = (int)c.m; a.N = (int)c.n; a.K = (int)c.k;
     a.MB = (int)((c.m + 15) / 16 * 16);
     a.np = c.x1 ? 2 : 1;
-    a.tiles = (int)((c.n + BM - 1) / BM);
     a.w_static = c.w_static ? 1 : 0;
     if (int rc = wait_ctx(&a.wait)) return rc;
     const int num_kb = (int)((c.k + BK - 1) / BK), sms = sm_count();
-    const long long units = (long long)a.tiles * (long long)c.batch;
+    const long long units = (long long)((c.n + BM - 1) / BM);
     const int stage = BM * BKB + a.np * a.MB * BKB;
     // The most ranges of k (a power of two: clusters of 3, 5, ... pack badly) whose CTAs all find a place at once, with two
     // stages each at least.  e4m3, 32 rows, us
@@ -303,11 +298,11 @@ int launch(const SkinnyCall &c, cudaStream_t st) {
     a.nstage = nstage > SK_MAX_STAGES ? SK_MAX_STAGES : nstage;
     a.S = S;
     CUtensorMap mw, mx0, mx1;
-    int rc = MN ? make_map_mn(&mw, c.w, c.n, c.k, c.ldw, c.batch, c.w_bs, &a.w_inner)
-                : make_map3(&mw, c.w, ELEM, c.n, c.k, c.ldw, BM, c.batch, c.w_bs, &a.w_inner);
+    int inner;  // one matrix each: the order (k, rows, 1)
+    int rc = MN ? make_map_mn(&mw, c.w, c.n, c.k, c.ldw, 1, 0, &inner) : make_map3(&mw, c.w, ELEM, c.n, c.k, c.ldw, BM, 1, 0, &inner);
     if (rc) return rc;
-    if ((rc = make_map3(&mx0, c.x0, ELEM, c.m, c.k, c.ldx, a.MB, c.batch, c.x_bs, &a.x_inner))) return rc;
-    if ((rc = make_map3(&mx1, c.x1 ? c.x1 : c.x0, ELEM, c.m, c.k, c.ldx, a.MB, c.batch, c.x_bs, &a.x_inner))) return rc;
+    if ((rc = make_map3(&mx0, c.x0, ELEM, c.m, c.k, c.ldx, a.MB, 1, 0, &inner))) return rc;
+    if ((rc = make_map3(&mx1, c.x1 ? c.x1 : c.x0, ELEM, c.m, c.k, c.ldx, a.MB, 1, 0, &inner))) return rc;
     // never less than what keeps a third CTA off the SM: two of them may hold all of its tensor memory
     size_t smem = (size_t)a.nstage * stage + red + 1024;
     const size_t out = (size_t)a.MB * BM * sizeof(float) + 1024;  // a single CTA's rows, over the drained ring
@@ -363,15 +358,14 @@ bool gemm_skinny_wanted(size_t m, size_t n, size_t k_bytes, int pieces) {
 // y bf16 [m, n] = x_scale[m] * w_scale[n] * (x_hi (+ x_lo)) * wq^T, all operands row-major e4m3.  wq is a static weight.
 int launch_skinny_fp8(void *y, const uint8_t *x_hi, const uint8_t *x_lo, const float *x_scale, const uint8_t *wq,
                       const float *w_scale, size_t m, size_t n, size_t k, size_t ldy, cudaStream_t st) {
-    const SkinnyCall c{y, x_hi, x_lo, wq, nullptr, x_scale, w_scale, m, n, k, k, k, ldy, 1, 0, 0, 0, true};
+    const SkinnyCall c{y, x_hi, x_lo, wq, nullptr, x_scale, w_scale, m, n, k, k, k, ldy, true};
     return launch<0, false>(c, st);
 }
 
-// 16-bit operands; w_mn: rhs is [k, n] with n contiguous.  lhs_bs / rhs_bs / dst_bs: elements between batch entries.
+// 16-bit operands; w_mn: rhs is [k, n] with n contiguous.
 int launch_skinny_16bit(xn_dtype dt, void *dst, const void *lhs, const void *rhs, const void *bias, size_t m, size_t n, size_t k,
-                        size_t lda, size_t ldb, size_t ldd, size_t batch, size_t lhs_bs, size_t rhs_bs, size_t dst_bs, bool w_mn,
-                        cudaStream_t st) {
-    const SkinnyCall c{dst, lhs, nullptr, rhs, bias, nullptr, nullptr, m, n, k, lda, ldb, ldd, batch, lhs_bs, rhs_bs, dst_bs, rhs_is_static()};
+                        size_t lda, size_t ldb, size_t ldd, bool w_mn, cudaStream_t st) {
+    const SkinnyCall c{dst, lhs, nullptr, rhs, bias, nullptr, nullptr, m, n, k, lda, ldb, ldd, rhs_is_static()};
     if (dt == XN_BF16) return w_mn ? launch<1, true>(c, st) : launch<1, false>(c, st);
     return w_mn ? launch<2, true>(c, st) : launch<2, false>(c, st);
 }

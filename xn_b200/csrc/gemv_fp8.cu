@@ -1,4 +1,4 @@
-// fp8-e4m3 weight linear for decode-sized batches (M <= 16 per pass): weight streaming with the
+// fp8-e4m3 weight linear for decode-sized batches (M <= 8): weight streaming with the
 // weights used as stored -- no dequantization instructions at all.  No counterpart in the
 // reference; contract in include/xn_mm.h.
 //
@@ -8,7 +8,7 @@
 // per lane feeds two MMAs directly: the MMA's k positions are a fixed permutation of memory order,
 // applied identically to the activation fragment, which shared memory serves as one 128-bit read
 // of 16 contiguous bytes of the activation row.  Output rows ride the MMA's 16-row dimension; the
-// activation rows its 8 columns (two column groups for M = 9..16).
+// activation rows its 8 columns.
 //
 // Schedule.  `tpc` consecutive 16-row tiles per CTA (about one CTA per SM), `ksplit` warps per tile
 // reduced in a fixed order.  Every warp keeps DEPTH 64-byte k steps (two 128-bit loads each) in
@@ -43,7 +43,7 @@ __device__ __forceinline__ void cp_async16(void *smem_dst, const void *gsrc, boo
 // rows a quarter-warp reads fall in distinct 16-byte bank groups
 __host__ __device__ inline int x_row_stride(int kc) { return (kc + 127) / 128 * 128 + 64; }
 
-template <int MT, bool LO>
+template <bool LO>
 __global__ void __launch_bounds__(MAX_WARPS * 32, 1)
 linear_fp8_gemv_kernel(__nv_bfloat16 *__restrict__ y, const uint8_t *__restrict__ x_hi,
                        const uint8_t *__restrict__ x_lo, const float *__restrict__ x_scale,
@@ -52,8 +52,8 @@ linear_fp8_gemv_kernel(__nv_bfloat16 *__restrict__ y, const uint8_t *__restrict_
     extern __shared__ __align__(16) unsigned char smem[];
     const int RS = x_row_stride(kchunk);
     unsigned char *sHi = smem;
-    unsigned char *sLo = smem + (size_t)MT * 8 * RS;
-    float *red = reinterpret_cast<float *>(smem + (size_t)(LO ? 2 : 1) * MT * 8 * RS);
+    unsigned char *sLo = smem + (size_t)8 * RS;
+    float *red = reinterpret_cast<float *>(smem + (size_t)(LO ? 2 : 1) * 8 * RS);
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -62,15 +62,11 @@ linear_fp8_gemv_kernel(__nv_bfloat16 *__restrict__ y, const uint8_t *__restrict_
     const bool valid = tile < tiles;
     const size_t r0 = valid ? min((size_t)tile * 16 + g, n - 1) : 0, r1 = valid ? min((size_t)tile * 16 + g + 8, n - 1) : 0;
 
-    float acc[MT][4];
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[mt][i] = 0.0f;
+    float acc[4] = {};
     // scales of what this lane stores at the end, requested early.  Those of the rows by the storing warps only: the load is
     // coherent and so served by L2, where every warp of every CTA would ask for the same sector (8 x 2560 x 4096 7.1 us
     // against 6.8).
-    float xs_reg[MT][2] = {}, ws_reg[2];
+    float xs_reg[2] = {}, ws_reg[2];
 
     for (int kc0 = 0; kc0 < k; kc0 += kchunk) {
         const int kc = min(kchunk, k - kc0);
@@ -97,20 +93,16 @@ linear_fp8_gemv_kernel(__nv_bfloat16 *__restrict__ y, const uint8_t *__restrict_
             asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
             if (ks == 0)
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const int row_m = 8 * mt + 2 * t + e;
-                        if (row_m < m) xs_reg[mt][e] = ld_act_f32(x_scale + row_m);
-                    }
+                for (int e = 0; e < 2; ++e)
+                    if (2 * t + e < m) xs_reg[e] = ld_act_f32(x_scale + 2 * t + e);
             ws_reg[0] = valid ? __ldg(w_scale + r0) : 0.0f;
             ws_reg[1] = valid ? __ldg(w_scale + r1) : 0.0f;
         } else {
             __syncthreads();  // every warp is done with the previous chunk's pieces
         }
-        // stage rows [0, 8*MT) x bytes [kc0, kc0 + round64(kc)) of both pieces, zero-filled outside
+        // stage rows [0, 8) x bytes [kc0, kc0 + round64(kc)) of both pieces, zero-filled outside
         const int cols16 = (kc + 63) / 64 * 4;
-        for (int idx = tid; idx < MT * 8 * cols16; idx += blockDim.x) {
+        for (int idx = tid; idx < 8 * cols16; idx += blockDim.x) {
             const int row = idx / cols16, c = idx % cols16;
             const bool ok = row < m && c * 16 < kc;
             const size_t src = ok ? (size_t)row * k + kc0 + c * 16 : 0;
@@ -125,16 +117,13 @@ linear_fp8_gemv_kernel(__nv_bfloat16 *__restrict__ y, const uint8_t *__restrict_
             for (int i = 0; i < DEPTH; ++i) {
                 if (st + i < st1) {
                     const int off = (st + i) * 64 + 16 * t;
-#pragma unroll
-                    for (int mt = 0; mt < MT; ++mt) {
-                        const uint4 bh = *reinterpret_cast<const uint4 *>(sHi + (size_t)(8 * mt + g) * RS + off);
-                        mma_e4m3(acc[mt], w0[i].x, w1[i].x, w0[i].y, w1[i].y, bh.x, bh.y);
-                        mma_e4m3(acc[mt], w0[i].z, w1[i].z, w0[i].w, w1[i].w, bh.z, bh.w);
-                        if (LO) {
-                            const uint4 bl = *reinterpret_cast<const uint4 *>(sLo + (size_t)(8 * mt + g) * RS + off);
-                            mma_e4m3(acc[mt], w0[i].x, w1[i].x, w0[i].y, w1[i].y, bl.x, bl.y);
-                            mma_e4m3(acc[mt], w0[i].z, w1[i].z, w0[i].w, w1[i].w, bl.z, bl.w);
-                        }
+                    const uint4 bh = *reinterpret_cast<const uint4 *>(sHi + (size_t)g * RS + off);
+                    mma_e4m3(acc, w0[i].x, w1[i].x, w0[i].y, w1[i].y, bh.x, bh.y);
+                    mma_e4m3(acc, w0[i].z, w1[i].z, w0[i].w, w1[i].w, bh.z, bh.w);
+                    if (LO) {
+                        const uint4 bl = *reinterpret_cast<const uint4 *>(sLo + (size_t)g * RS + off);
+                        mma_e4m3(acc, w0[i].x, w1[i].x, w0[i].y, w1[i].y, bl.x, bl.y);
+                        mma_e4m3(acc, w0[i].z, w1[i].z, w0[i].w, w1[i].w, bl.z, bl.w);
                     }
                 }
                 load(i, st + i + DEPTH);
@@ -147,31 +136,25 @@ linear_fp8_gemv_kernel(__nv_bfloat16 *__restrict__ y, const uint8_t *__restrict_
         __syncthreads();
         if (ks > 0)
 #pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) red[((size_t)warp * MT * 4 + mt * 4 + i) * 32 + lane] = acc[mt][i];
+            for (int i = 0; i < 4; ++i) red[((size_t)warp * 4 + i) * 32 + lane] = acc[i];
         __syncthreads();
         if (ks == 0)
             for (int o = 1; o < ksplit; ++o)
 #pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) acc[mt][i] += red[((size_t)(warp + o) * MT * 4 + mt * 4 + i) * 32 + lane];
+                for (int i = 0; i < 4; ++i) acc[i] += red[((size_t)(warp + o) * 4 + i) * 32 + lane];
     }
     if (ks == 0 && valid) {
 #pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const size_t row_n = (size_t)tile * 16 + g + 8 * (i >> 1);
-                const int row_m = 8 * mt + 2 * t + (i & 1);
-                if (row_n < n && row_m < m)
-                    y[(size_t)row_m * n + row_n] = __float2bfloat16_rn(ws_reg[i >> 1] * (xs_reg[mt][i & 1] * acc[mt][i]));
-            }
+        for (int i = 0; i < 4; ++i) {
+            const size_t row_n = (size_t)tile * 16 + g + 8 * (i >> 1);
+            const int row_m = 2 * t + (i & 1);
+            if (row_n < n && row_m < m)
+                y[(size_t)row_m * n + row_n] = __float2bfloat16_rn(ws_reg[i >> 1] * (xs_reg[i & 1] * acc[i]));
+        }
     }
 }
 
-template <int MT, bool LO>
+template <bool LO>
 int launch(__nv_bfloat16 *y, const uint8_t *x_hi, const uint8_t *x_lo, const float *x_scale, const uint8_t *wq,
            const float *w_scale, int m, size_t n, int k, cudaStream_t st) {
     const int tiles = (int)((n + 15) / 16);
@@ -182,15 +165,15 @@ int launch(__nv_bfloat16 *y, const uint8_t *x_hi, const uint8_t *x_lo, const flo
     // largest k chunk (multiple of 128) whose staged pieces fit the shared-memory budget
     const int pieces = LO ? 2 : 1;
     int kchunk = (k + 127) / 128 * 128;
-    while ((size_t)pieces * MT * 8 * x_row_stride(kchunk) > (size_t)SMEM_BUDGET - MAX_WARPS * MT * 4 * 32 * 4)
+    while ((size_t)pieces * 8 * x_row_stride(kchunk) > (size_t)SMEM_BUDGET - MAX_WARPS * 4 * 32 * 4)
         kchunk = ((kchunk / 128 + 1) / 2) * 128;
     const int nst = ((kchunk < k ? kchunk : k) + 63) / 64;
     if (ksplit > nst / DEPTH) ksplit = nst / DEPTH;
     if (ksplit < 1) ksplit = 1;
     const int warps = tpc * ksplit;
     const int grid = (tiles + tpc - 1) / tpc;
-    const size_t smem = (size_t)pieces * MT * 8 * x_row_stride(kchunk) + (size_t)warps * MT * 4 * 32 * sizeof(float);
-    auto kern = linear_fp8_gemv_kernel<MT, LO>;
+    const size_t smem = (size_t)pieces * 8 * x_row_stride(kchunk) + (size_t)warps * 4 * 32 * sizeof(float);
+    auto kern = linear_fp8_gemv_kernel<LO>;
     XN_ENSURE_SMEM(kern, smem);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
@@ -212,8 +195,8 @@ int launch(__nv_bfloat16 *y, const uint8_t *x_hi, const uint8_t *x_lo, const flo
 int launch_linear_fp8_gemv(void *y, const uint8_t *x_hi, const uint8_t *x_lo, const float *x_scale,
                            const uint8_t *wq, const float *w_scale, int m, size_t n, int k, cudaStream_t st) {
     __nv_bfloat16 *yy = (__nv_bfloat16 *)y;
-    return x_lo ? launch<1, true>(yy, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st)
-                : launch<1, false>(yy, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st);
+    return x_lo ? launch<true>(yy, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st)
+                : launch<false>(yy, x_hi, x_lo, x_scale, wq, w_scale, m, n, k, st);
 }
 
 }  // namespace xn
