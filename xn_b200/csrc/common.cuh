@@ -212,7 +212,7 @@ int launch_gemv_dense(xn_dtype dt, void *dst, const void *lhs, const void *rhs, 
                       cudaStream_t st);
 bool gemm_skinny_wanted(size_t m, size_t n, size_t k_bytes, int pieces);
 int split_rows_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_scale, const void *x, xn_dtype dtype, size_t m, size_t k, bool early,
-                    bool dependent, void *stream);
+                    void *stream);
 int launch_skinny_fp8(void *y, const uint8_t *x_hi, const uint8_t *x_lo, const float *x_scale, const uint8_t *wq,
                       const float *w_scale, size_t m, size_t n, size_t k, size_t ldy, cudaStream_t st);
 int launch_skinny_16bit(xn_dtype dt, void *dst, const void *lhs, const void *rhs, const void *bias, size_t m, size_t n, size_t k,

@@ -1391,7 +1391,7 @@ int decode_attention_impl(void *out_bf16, const void *q_bf16, size_t q_batch_str
         XN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, decode_attention_combine_kernel, (__nv_bfloat16 *)out_bf16,
                                          (const float *)workspace, splits));
     }
-    if (x_hi) return split_rows_e4m3(x_hi, x_lo, x_scale, out_bf16, XN_BF16, batch, heads * head_dim, true, true, stream);
+    if (x_hi) return split_rows_e4m3(x_hi, x_lo, x_scale, out_bf16, XN_BF16, batch, heads * head_dim, true, stream);
     return XN_OK;
 }
 }  // namespace
@@ -1512,7 +1512,7 @@ extern "C" int xn_mm_decode_attention_append_e4m3(uint8_t *x_hi, uint8_t *x_lo, 
     cfg.blockDim = dim3(HD);
     XN_CHECK_CUDA(cudaLaunchKernelEx(&cfg, decode_attention_combine_kernel, (__nv_bfloat16 *)out_bf16, (const float *)workspace,
                                      splits));
-    if (x_hi) return split_rows_e4m3(x_hi, x_lo, x_scale, out_bf16, XN_BF16, batch, heads * head_dim, true, true, stream);
+    if (x_hi) return split_rows_e4m3(x_hi, x_lo, x_scale, out_bf16, XN_BF16, batch, heads * head_dim, true, stream);
     return XN_OK;
 }
 

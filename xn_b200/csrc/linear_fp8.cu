@@ -28,6 +28,8 @@ static inline bool fp8_gemv_wanted(size_t m, size_t n, size_t k, bool two_pieces
     return m <= 8 && (n * k < FP8_GEMV_MAX_WEIGHT || (!two_pieces && k <= 4096 && n * k < FP8_GEMV_MAX_WEIGHT_ONE_PIECE));
 }
 
+static constexpr size_t FP8_SPLIT_EARLY_WEIGHT = 8u << 20;
+
 static inline size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 }  // namespace xn
 
@@ -106,10 +108,13 @@ extern "C" int xn_mm_linear_fp8(void *y_bf16, const void *x_bf16, const uint8_t 
     uint8_t *hi = (uint8_t *)workspace;
     uint8_t *lo = hi + round_up(m * k, 256);
     float *xs = (float *)(lo + round_up(m * k, 256));
-    // The streaming kernels fetch weights while the split runs.  The tiled kernel fetches nothing before its wait: let in early it
-    // only stands in the split's way, and the split in the previous call's (W8A16 250 x 12288 x 4096 33.4 us, 32.8 in plain order).
-    const bool streams = fp8_gemv_wanted(m, n, k, variant == 0) || gemm_skinny_wanted(m, n, k, variant == 0 ? 2 : 1);
-    int rc = split_rows_e4m3(hi, variant == 0 ? lo : nullptr, xs, x_bf16, XN_BF16, m, k, streams, streams, stream);
+    // The streaming kernels fetch weights while the split runs, and a small product gains from any overlap.  The tiled kernel
+    // fetches nothing before its wait; let in beside the split, a long run of calls at the power cap loses by it.  us in such a
+    // run, let in early / not / split in plain order: W8A16 250 x 12288 x 4096 33.5 / 33.0 / 32.8, 1000 x 4096 x 4096 36.6 / 35.9 / 36.8,
+    // W8A8 500 x 12288 x 4096 37.7 / 36.8 / 37.1, 250 x 1024 x 1024 7.5 / 8.0 / 9.2.
+    const int pieces = variant == 0 ? 2 : 1;
+    const bool early = fp8_gemv_wanted(m, n, k, pieces == 2) || gemm_skinny_wanted(m, n, k, pieces) || n * k < FP8_SPLIT_EARLY_WEIGHT;
+    int rc = split_rows_e4m3(hi, variant == 0 ? lo : nullptr, xs, x_bf16, XN_BF16, m, k, early, stream);
     if (rc) return rc;
     return xn_mm_linear_fp8_pieces(y_bf16, hi, variant == 0 ? lo : nullptr, xs, wq, w_scale, m, n, k, stream);
 }
@@ -188,7 +193,7 @@ extern "C" int xn_mm_linear_fp8_noalloc(void *y_bf16, const void *x_bf16, const 
     uint8_t *hi = base;
     uint8_t *lo = base + NOALLOC_MAX_ELEMS;
     float *xs = reinterpret_cast<float *>(base + NOALLOC_SCALE_OFFSET);
-    rc = split_rows_e4m3(hi, variant == 0 ? lo : nullptr, xs, x_bf16, XN_BF16, m, k, true, true, stream);
+    rc = split_rows_e4m3(hi, variant == 0 ? lo : nullptr, xs, x_bf16, XN_BF16, m, k, true, stream);
     if (rc) return rc;
     // Up to 64 rows no kernel needs scratch of its own: the tensor-memory kernel's split tiles meet in shared memory.
     return xn_mm_linear_fp8_pieces(y_bf16, hi, variant == 0 ? lo : nullptr, xs, wq, w_scale, m, n, k, stream);

@@ -326,10 +326,9 @@ extern "C" int xn_mm_quantize_weights_fp8(uint8_t *wq, float *w_scale, const voi
 }
 
 // `early`: the next kernel may begin while this one runs -- for pieces that are this library's own activations; a caller's have the
-// layout of an fp8 weight and may be used as one (see dependent_begin).  `dependent`: this kernel may itself begin beside the
-// previous one.
+// layout of an fp8 weight and may be used as one (see dependent_begin).
 int xn::split_rows_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_scale, const void *x, xn_dtype dtype, size_t m, size_t k, bool early,
-                        bool dependent, void *stream) {
+                        void *stream) {
     XN_REQUIRE(valid_dtype(dtype), "split_rows_e4m3: unknown dtype %d", (int)dtype);
     if (m == 0 || k == 0) return XN_OK;
     XN_REQUIRE(x_hi && x_scale && x, "split_rows_e4m3: null pointer");
@@ -342,7 +341,7 @@ int xn::split_rows_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_scale, const void
             using T = std::remove_const_t<std::remove_pointer_t<decltype(p)>>;
             auto kern = early ? (small ? split_rows_e4m3_vec_kernel<T, 2, true> : split_rows_e4m3_vec_kernel<T, 8, true>)
                                     : (small ? split_rows_e4m3_vec_kernel<T, 2, false> : split_rows_e4m3_vec_kernel<T, 8, false>);
-            return launch_kernel(dependent, kern, dim3((unsigned)m), dim3(256), 0, st, x_hi, x_lo, x_scale, p, k);
+            return launch_dependent(kern, dim3((unsigned)m), dim3(256), 0, st, x_hi, x_lo, x_scale, p, k);
         };
         return dtype == XN_BF16 ? go((const __nv_bfloat16 *)x) : go((const __half *)x);
     }
@@ -355,5 +354,5 @@ int xn::split_rows_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_scale, const void
 extern "C" int xn_mm_split_rows_e4m3(uint8_t *x_hi, uint8_t *x_lo, float *x_scale, const void *x, xn_dtype dtype, size_t m, size_t k,
                                      void *stream) {
     XN_API_RANGE("xn_mm_split_rows_e4m3");
-    return xn::split_rows_e4m3(x_hi, x_lo, x_scale, x, dtype, m, k, false, true, stream);
+    return xn::split_rows_e4m3(x_hi, x_lo, x_scale, x, dtype, m, k, false, stream);
 }
