@@ -49,6 +49,14 @@ def test_int4_layer_takes_any_leading_dimensions(xn, cuda, shape):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float64, torch.int64, torch.int32, torch.int8, torch.uint8])
+def test_refused_types_are_named_as_torch_names_them(xn, cuda, dtype):
+    a = torch.zeros(4, 4, dtype=dtype, device=cuda)
+    with pytest.raises(xn.XnError, match=f"not supported for dtype {dtype}"):
+        xn.matmul_t(a, a)
+
+
+@pytest.mark.gpu
 def test_add_of_transposed_views(xn, cuda):
     a, b = torch.randn(37, 50, device=cuda), torch.randn(37, 50, device=cuda)
     for x, y in ((a.t(), b.t()), (a.t(), b.t().contiguous()), (a.t().contiguous(), b.t())):

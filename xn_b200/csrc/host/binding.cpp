@@ -81,7 +81,22 @@ void require_cuda(const at::Tensor &t) {
     if (!t.is_cuda()) raise_xn(XN_ERR_INVALID, "xn_b200 runs on CUDA tensors only; there is no CPU path");
 }
 
-const char *dtype_name(at::ScalarType s) { return c10::toString(s); }
+// as torch prints them
+const char *dtype_name(at::ScalarType s) {
+    switch (s) {
+        case at::kFloat: return "torch.float32";
+        case at::kHalf: return "torch.float16";
+        case at::kBFloat16: return "torch.bfloat16";
+        case at::kDouble: return "torch.float64";
+        case at::kLong: return "torch.int64";
+        case at::kInt: return "torch.int32";
+        case at::kShort: return "torch.int16";
+        case at::kChar: return "torch.int8";
+        case at::kByte: return "torch.uint8";
+        case at::kBool: return "torch.bool";
+        default: return c10::toString(s);
+    }
+}
 
 xn_dtype dtype_code(at::ScalarType s) {
     if (s == at::kFloat) return XN_F32;
