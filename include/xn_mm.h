@@ -16,14 +16,17 @@
  * xn-core/src/backend.rs:4).
  *
  * Library-owned device memory: buffers per (device, stream) that the library allocates when a stream first needs
- * them and grows when a larger problem arrives (cudaMalloc, i.e. not allowed during stream capture: run each shape
- * once before capturing it, as a decode loop does anyway; a stream under capture borrows the buffer of the stream
- * that ran those shapes, so keep the graph's replays ordered with that stream's own calls).  Calls on different
- * streams use different buffers and may overlap.  They hold the repacked operands of an f32 xn_mm_gemm with 17 or
- * more rows (three tf32 pieces per element: 12 bytes per operand element, refused above 2 GiB in favour of the plain
- * f32 kernel; XN_MM_F32_TC=0 in the environment keeps every f32 call on the plain kernel), unpacked block weights,
- * lhs rows copied to a pitch TMA can address, and the partial sums of output tiles that the tiled tensor-memory
- * kernel cuts along k (up to 76 MB; a captured launch, or one for which there is no memory, cuts none).
+ * them and grows, by half at least, when a larger problem arrives (cudaMalloc).  They hold what one launch of a call leaves
+ * for the next: the repacked operands of an f32 xn_mm_gemm with 17 or more rows (three tf32 pieces per element: 12 bytes
+ * per operand element, refused above 2 GiB in favour of the plain f32 kernel; XN_MM_F32_TC=0 in the environment keeps
+ * every f32 call on the plain kernel), unpacked block weights, lhs rows copied to a pitch TMA can address (at most 512
+ * MiB; larger ones take the any-stride kernel), and the partial sums of output tiles that the tiled tensor-memory kernel cuts
+ * along k (39 MB of them at most; without memory for them no tile is cut).  Calls on different streams use different buffers and may
+ * overlap; the launches of one call stay together on their stream, whichever host threads call.  Under stream
+ * capture the last two are blocks of the graph's own, which it keeps as long as it lives and which need no earlier call (copied
+ * rows up to 64 MiB); f32 operands and unpacked weights cannot be allocated then: run each such shape once before
+ * capturing it, the captured call borrows the buffer of the stream that ran it, so keep the graph's replays ordered with
+ * that stream's own calls.
  * Nothing else allocates;
  * xn_mm_linear_fp8_noalloc runs only kernels that need none of it.
  */
@@ -72,8 +75,8 @@ int xn_mm_abi_version(void);
  * Library-owned scratch (see the top of this file) is kept per (device, stream) for the life of the process;
  * a replaced block is kept too, since a captured graph may still point at it.  xn_mm_release_scratch
  * synchronises the current device and frees the blocks of `stream` (or of every stream when all_streams != 0)
- * together with all replaced blocks of the device; graphs captured earlier that ran a call which
- * uses them must not be replayed afterwards.
+ * together with all replaced blocks of the device and the blocks of graphs that are gone; graphs captured earlier that
+ * borrowed one of the former must not be replayed afterwards.
  * ------------------------------------------------------------------------------------------ */
 int xn_mm_device_status(unsigned *timeouts_out);
 int xn_mm_clear_device_status(void);
@@ -381,9 +384,8 @@ int xn_mm_kv_append2(xn_dtype dtype, void *k_cache, void *v_cache, const void *k
  * is looked up for the current device).  Every argument is checked before anything is enqueued, so a
  * rejected call leaves the shared array untouched.  A device-side wait that runs out inside this call is
  * still bounded, but it is reported to xn_mm_device_status only if some other entry point has already
- * set up the device's status word (this one must not allocate it).  It runs only kernels that need no scratch of their own (the
- * weight-streaming kernel up to 32 rows, the tiled tensor-memory kernel beyond), so from 9 rows on its
- * results can differ from xn_mm_linear_fp8 in the last bf16 bit (another summation order). */
+ * set up the device's status word (this one must not allocate it).  It runs the kernels of
+ * xn_mm_linear_fp8, which up to 64 rows need no scratch of their own: results are the same. */
 size_t xn_mm_linear_fp8_noalloc_max_elems(void);
 int xn_mm_linear_fp8_noalloc(void *y_bf16, const void *x_bf16, const uint8_t *wq, const float *w_scale,
                              size_t m, size_t n, size_t k, int variant, void *stream);

@@ -1,5 +1,5 @@
 """The tiled tensor-memory kernel with the tiles of its last, partly filled round cut along k: few tiles and many, ragged
-rows, columns and k, two row blocks per tile, both fp8 variants, a bias, batches, and a captured launch (which cuts none).
+rows, columns and k, two row blocks per tile, both fp8 variants, a bias, batches, and a captured launch.
 
 Bounds: as in test_few_rows_gpu.py, |y - ref| <= u |ref| + k 2^-23 sum|a||b| (the tensor cores add with truncation: one
 ulp per step instead of half) with one more u where a bias is added to the rounded product."""
@@ -34,7 +34,7 @@ def test_16bit(xn, cuda, dtype, m, n, k, bias):
     layer = xn.Linear(w, b)
     y = layer(x)
     _check(y, x, w, U[dtype], b)
-    for _ in range(3):  # the arrival counters are zero again, the sums run in a fixed order
+    for _ in range(3):  # the sums run in a fixed order
         assert torch.equal(layer(x), y)
 
 
